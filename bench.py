@@ -166,18 +166,21 @@ def make_ic(cfg, pl):
 PHASE_KERNELS = {
     "inv_y": "k_inv_y1", "inv_x": "k_inv_x", "inv_z": "k_inv_z", "z_products": "k_z_fused",
     "fwd_x": "k_fwd_x", "fwd_y": "k_fwd_y_pipe", "nl_assembly": "k_nl",
-    "rhs_nl": "k_rhs_tiles", "mean_systems": "k_zero_step", "substitution": "k_subst_tpb", "kstd_out": "k_kstd_tiles",
+    "rhs_nl": "k_rhs_tiles", "mean_systems": "k_zero_step", "substitution": "k_subst_block", "kstd_out": "k_kstd_tiles",
 }
 
 
-def phase_bytes(g, nsys, nact, T, ncls, Tc, kl, ku, stages, factor_bytes, factor_entries=0):
+def phase_bytes(g, nsys, nact, T, ncls, Tc, kl, ku, stages, factor_bytes, factor_entries=0, units=None):
     """Algorithmic HBM bytes of one launch of each phase (averaged over the
     stages): every array a phase must read from or write to HBM once.
     g: dict with NXH, NYA, NXA, NZ, NZA, nF (full variables), nQ (quadratic
     variables).  Transform intermediates are 16-byte complex where the data are
     complex (after an x r2c / before an x c2r) and 8-byte real otherwise.
     factor_entries: LU band entries per block that the substitution reads (the
-    entries nonzero in some block; 0 = the whole band, 2 kl + ku + 1 per column)."""
+    entries nonzero in some block; 0 = the whole band, 2 kl + ku + 1 per column);
+    units: LU factorisations held (None = one per active system), each read once
+    for all the systems that share it."""
+    units = nact if units is None else units
     NXH, NYA, NXA, NZ, NZA, nF, nQ = (g[k] for k in ("NXH", "NYA", "NXA", "NZ", "NZA", "nF", "nQ"))
     y1 = lambda nv: nv * NYA * NXH * NZ * 16   # [var][y][kx][n] complex
     y2 = lambda nv: nv * NYA * NXA * NZ * 8    # [var][y][x][n] real
@@ -205,13 +208,13 @@ def phase_bytes(g, nsys, nact, T, ncls, Tc, kl, ku, stages, factor_bytes, factor
     #     K_std out, in every stage but the last (which needs no K_std);
     #     whole systems: solution in, stage output and K_std out
     rhs = sub = kst = 0
-    nblk_cols = nact * ncls * Tc
+    nblk_cols, unit_cols = nact * ncls * Tc, units * ncls * Tc
     for i in range(stages):
         last = (i == stages - 1)
         rhs += (nsys * 16 * T * (1 + 2 * i + (0 if last else 1) + 1) + nact * 16 * nQ * NZ
                 + (nsys - nact) * 16 * T * (0 if last else 1))
-        entries = factor_entries * nact * ncls if factor_entries else nblk_cols * (2 * kl + ku + 1)
-        sub += entries * factor_bytes + nblk_cols + 4 * 16 * nblk_cols
+        entries = factor_entries * units * ncls if factor_entries else unit_cols * (2 * kl + ku + 1)
+        sub += entries * factor_bytes + unit_cols + 4 * 16 * nblk_cols
         kst += 16 * nblk_cols + nact * 16 * T * (1 if last else 2)
     out["rhs_nl"] = rhs / stages
     out["substitution"] = sub / stages
@@ -448,7 +451,8 @@ def run_ours(args, cfg):
     geo = {"NXH": pl.NXH, "NYA": pl.NYAA, "NXA": pl.NXAA, "NZ": pl.NZ, "NZA": pl.NZAA,
            "nF": pl.query(8), "nQ": pl.query(9)}
     fentries = pl.query(1200)  # after the factorisation of the timed steps
-    pbytes = phase_bytes(geo, nsys, nact, T, ncls, Tc, kl_c, ku_c, pl.stages, fbytes, fentries)
+    pbytes = phase_bytes(geo, nsys, nact, T, ncls, Tc, kl_c, ku_c, pl.stages, fbytes, fentries,
+                         units=pl.query(1300))
     peak, src = read_peaks()
     phases = {}
     nlaunch = phase_launches(pl.stages, ncls)

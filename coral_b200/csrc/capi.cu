@@ -93,9 +93,16 @@ struct KSys {
   int *row_pos = nullptr, *col_pos = nullptr, *cls_row = nullptr, *cls_col = nullptr;
   unsigned char* colflip_cls = nullptr;
   DevEll Lp;
-  // per class column, band entries nonzero in any block (thread-per-block layout)
+  // block layout of a split system (SolveArgs::work2): factorisation units, each
+  // shared by the (kx, ky) and (kx, -ky) systems of a recipe with that symmetry
+  int upw = 32, ngrp = 0, nunit = 0;
+  int *slot = nullptr, *lane_sid = nullptr, *unit_sid = nullptr;
+  unsigned char *row_neg = nullptr, *col_neg = nullptr;
   unsigned long long* cmask = nullptr;
-  unsigned *lmask = nullptr, *umask = nullptr;
+  double *lpack = nullptr, *upack = nullptr;
+  uint4* finfo = nullptr;
+  uint4* binfo = nullptr;
+  int* ptot = nullptr;
   // operator-stationary K_std: tile windows and window-relative L
   int* tile_win = nullptr;
   int tile_lwin_max = 0;
@@ -105,7 +112,7 @@ struct KSys {
   DevEll Mw, NLw;
   DevGEll NLg;
   double2* work = nullptr;
-  double2* work2 = nullptr;  // thread-per-block layout of the active systems' vectors (split only)
+  double2* work2 = nullptr;  // block layout of the active systems' vectors (split only)
   std::vector<std::vector<int>> tab_t;   // per var: [NZ][kTabW]
   std::vector<std::vector<double>> tab_v;
   std::vector<int*> d_tab_t;
@@ -714,9 +721,7 @@ void setup(coral_handle* h, const std::string& eqs, const std::string& pars, con
       k.ku_s = k.ops.ku_cls;
       k.ldab_s = 2 * k.kl_s + k.ku_s + 1;
       k.ldab_s += k.ldab_s & 1;
-      k.wst = std::max(k.T, 2 * k.Tc);
-      k.work = mem.get<double2>(nsys * k.wst);  // never aliases aux: k_kstd_out gathers from it into aux
-      CK(cudaMemset(k.work, 0, nsys * k.wst * sizeof(double2)));
+      k.work = nullptr;  // the vectors are in work2
       k.row_pos = mem.upload(k.ops.row_cls_pos);
       k.col_pos = mem.upload(k.ops.col_cls_pos);
       k.cls_row = mem.upload(k.ops.cls_row);
@@ -810,15 +815,49 @@ void setup(coral_handle* h, const std::string& eqs, const std::string& pars, con
       k.NLg = upload_gell(mem, nw);
     }
     if (k.ncls == 2) {
-      // thread-per-block layouts: groups of 32 blocks (block = 2 act + class) side by side
-      const size_t ngroups = ((size_t)h->nact * 2 + 31) / 32;
-      k.abr = mem.get<double>(ngroups * k.Tc * k.ldab_s * 32);
-      k.dpiv = mem.get<unsigned char>(ngroups * k.Tc * 32);
-      k.work2 = mem.get<double2>(ngroups * k.Tc * 32);
-      k.cmask = mem.get<unsigned long long>(k.Tc);
-      k.lmask = mem.get<unsigned>(k.Tc);
-      k.umask = mem.get<unsigned>(k.Tc);
-      CK(cudaMemset(k.work2, 0, ngroups * k.Tc * 32 * sizeof(double2)));
+      // block layout: units in (kx, ky) order; with the mirror symmetry the
+      // systems (kx, ky > 0) and (kx, -ky) are one unit, lanes u and u + 16
+      const bool mirror = k.ops.ky_mirror && std::getenv("CORAL_NO_KY_MIRROR") == nullptr;
+      std::vector<int> slot(nsys, -1), lane_sid, unit_sid;
+      k.upw = mirror ? 16 : 32;
+      for (int ix = 0; ix < g.NXH; ++ix)
+        for (int iy = 0; iy < g.NYAA; ++iy) {
+          const int sid = ix * g.NYAA + iy, iym = (g.NYAA - iy) % g.NYAA, sidm = ix * g.NYAA + iym;
+          if (act_index[sid] < 0 || slot[sid] >= 0) continue;
+          const int u = (int)unit_sid.size(), lane = u / k.upw * 32 + u % k.upw;
+          unit_sid.push_back(sid);
+          if ((size_t)lane / 32 * 32 + 32 > lane_sid.size()) lane_sid.resize((size_t)lane / 32 * 32 + 32, -1);
+          slot[sid] = lane;
+          lane_sid[lane] = sid;
+          if (mirror && sidm != sid && act_index[sidm] >= 0 && g.ky[iym] == -g.ky[iy]) {
+            slot[sidm] = (lane + 16) | kMirrorBit;
+            lane_sid[lane + 16] = sidm;
+          }
+        }
+      k.nunit = (int)unit_sid.size();
+      k.ngrp = (int)(lane_sid.size() / 32);
+      k.slot = mem.upload(slot);
+      k.lane_sid = mem.upload(lane_sid);
+      k.unit_sid = mem.upload(unit_sid);
+      k.row_neg = mem.upload(k.ops.row_neg);
+      k.col_neg = mem.upload(k.ops.col_neg);
+      const size_t ng = 2 * (size_t)k.ngrp, cols = ng * k.Tc, kv = (size_t)k.kl_s + k.ku_s;
+      k.abr = mem.get<double>(cols * k.ldab_s * k.upw);
+      k.lpack = mem.get<double>(cols * std::max(k.kl_s, 1) * k.upw);
+      k.upack = mem.get<double>(cols * (kv + 1) * k.upw);
+      k.dpiv = mem.get<unsigned char>(cols * k.upw);
+      k.work2 = mem.get<double2>(cols * 32);
+      k.cmask = mem.get<unsigned long long>(2 * (size_t)k.Tc);
+      k.finfo = mem.get<uint4>(2 * (size_t)k.Tc);
+      k.binfo = mem.get<uint4>(2 * (size_t)k.Tc);
+      k.ptot = mem.get<int>(4);
+      // padding lanes have factors of their own (zeros) and zero right-hand sides
+      CK(cudaMemset(k.work2, 0, cols * 32 * sizeof(double2)));
+      CK(cudaMemset(k.dpiv, 0, cols * k.upw));
+      for (int c = 0; c < 2; ++c) {
+        const size_t last = (size_t)c * k.ngrp + k.ngrp - 1, n = (size_t)k.Tc * k.ldab_s * k.upw;
+        if (k.ngrp > 0) CK(cudaMemset(k.abr + last * n, 0, n * sizeof(double)));
+      }
     } else {
       if (k.real) k.abr = mem.get<double>((size_t)h->nact * k.Tc * k.ldab_s);
       else k.ab = mem.get<double2>((size_t)h->nact * k.T * k.ldab);
@@ -1165,10 +1204,16 @@ SolveArgs make_solve_args(coral_handle* h, KSys& k, int i, double dt) {
   sa.colflip_cls = k.colflip_cls;
   sa.Lp = k.Lp;
   sa.work2 = k.work2;
-  sa.nblk = k.ncls * h->nact;
-  sa.cls_col = k.cls_col;
-  sa.lmask = k.lmask;
-  sa.umask = k.umask;
+  sa.upw = k.upw;
+  sa.ngrp = k.ngrp;
+  sa.slot = k.slot;
+  sa.lane_sid = k.lane_sid;
+  sa.row_neg = k.row_neg;
+  sa.lpack = k.lpack;
+  sa.upack = k.upack;
+  sa.finfo = k.finfo;
+  sa.binfo = k.binfo;
+  sa.ptot = k.ptot;
   sa.tile_win = k.tile_win;
   sa.tile_lwin_max = k.tile_lwin_max;
   sa.rhs_win = k.rhs_win;
@@ -1457,14 +1502,21 @@ void factorize(coral_handle* h, double dt) {
     fa.col_pos = k.col_pos;
     fa.tpb = k.work2 != nullptr;
     fa.window = h->tune.factor_window;
+    fa.upw = k.upw;
+    fa.ngrp = k.ngrp;
     fa.cmask = k.cmask;
-    fa.lmask = k.lmask;
-    fa.umask = k.umask;
-    fa.nact = h->nact;
+    fa.lpack = k.lpack;
+    fa.upack = k.upack;
+    fa.finfo = k.finfo;
+    fa.binfo = k.binfo;
+    fa.ptot = k.ptot;
+    fa.cls_col = k.cls_col;
+    fa.col_neg = k.col_neg;
+    fa.nact = fa.tpb ? k.nunit : h->nact;
     fa.M = k.M;
     fa.L = k.L;
     fa.zsca = zsca;
-    fa.act_list = h->d_act_list;
+    fa.act_list = fa.tpb ? k.unit_sid : h->d_act_list;
     fa.ab = k.ab;
     fa.dpiv = k.dpiv;
     fa.kx = h->d_kx;
@@ -2201,15 +2253,17 @@ int coral_query(const coral_handle* hc, int what, long long* value) {
   if (base == CORAL_Q_SYS_FACTOR_ENTRIES && i < (int)h->ks.size()) {
     const KSys& k = h->ks[i];
     *value = 0;
-    if (!k.lmask || h->dt_factored < 0.0) return 0;
-    std::vector<unsigned> lm(k.Tc), um(k.Tc);
+    if (!k.ptot || h->dt_factored < 0.0) return 0;
+    int tot[4];
     if (cudaSetDevice(h->device) != cudaSuccess || cudaStreamSynchronize(h->stream) != cudaSuccess ||
-        cudaMemcpy(lm.data(), k.lmask, k.Tc * sizeof(unsigned), cudaMemcpyDeviceToHost) != cudaSuccess ||
-        cudaMemcpy(um.data(), k.umask, k.Tc * sizeof(unsigned), cudaMemcpyDeviceToHost) != cudaSuccess)
+        cudaMemcpy(tot, k.ptot, sizeof(tot), cudaMemcpyDeviceToHost) != cudaSuccess)
       return CORAL_ECUDA;
-    long long n = 0;
-    for (int j = 0; j < k.Tc; ++j) n += 1 + __builtin_popcount(lm[j]) + __builtin_popcount(um[j]);
+    const long long n = ((long long)tot[0] + tot[1] + tot[2] + tot[3] + 1) / 2;  // mean of the two classes
     *value = n;
+    return 0;
+  }
+  if (base == CORAL_Q_SYS_FACTOR_UNITS && i < (int)h->ks.size()) {
+    *value = h->ks[i].work2 ? h->ks[i].nunit : h->nact;
     return 0;
   }
   return CORAL_EBADARG;
@@ -2733,7 +2787,7 @@ int coral_run(coral_handle* h, int nsteps, const char* output_directory) {
 // and recipes) advanced together on one stream, one CUDA graph per step.  Per
 // stage every member's transforms and right-hand sides are queued, then the
 // band substitutions of all members run as one persistent launch
-// (k_subst_tpb_multi), then every member's K_std and mean systems.  The
+// (k_subst_block_multi), then every member's K_std and mean systems.  The
 // reference solves its systems one (kx, ky) at a time in a loop
 // (src/plane_layer/PL_algebra_z_3D.f90:197-214) and runs one problem per job.
 // ---------------------------------------------------------------------------
@@ -2746,9 +2800,10 @@ struct coral_ensemble {
   double graph_dt = -1.0;
   bool batched = false;                       // all members' substitutions in one launch
   std::vector<SolveArgs*> d_args;             // per stage: SolveArgs of every (member, system)
-  std::vector<long long*> d_prefix;           // per stage: first block of each (member, system)
+  std::vector<int*> d_prefix;                 // per stage: first group of each (member, system)
   std::vector<int> nsub;                      // per stage: (member, system) entries
-  std::vector<long long> total;               // per stage: blocks in all
+  std::vector<int> total;                     // per stage: groups in all
+  bool wide = false;                          // some member's groups have 32 units
   long long launches = 0;
   int launches_per_step = 0;
   // members' own phases run on these streams (member m on stream m mod kEnsStreams),
@@ -2804,24 +2859,25 @@ void ens_build_args(coral_ensemble* e, double dt) {
   e->batched = true;
   for (int i = 0; i < S && e->batched; ++i) {
     std::vector<SolveArgs> args;
-    std::vector<long long> prefix(1, 0);
+    std::vector<int> prefix(1, 0);
     for (coral_handle* h : e->mem)
       for (auto& k : h->ks) {
         if (!k.real) { e->batched = false; break; }
         SolveArgs sa = make_solve_args(h, k, i, dt);
         if (!subst_multi_supported(sa)) { e->batched = false; break; }
         args.push_back(sa);
-        prefix.push_back(prefix.back() + sa.nblk);
+        prefix.push_back(prefix.back() + sa.ncls * sa.ngrp);
+        e->wide = e->wide || sa.upw == 32;
       }
     if (!e->batched) break;
     SolveArgs* da = nullptr;
-    long long* dp = nullptr;
+    int* dp = nullptr;
     CK(cudaMalloc(&da, args.size() * sizeof(SolveArgs)));
     e->d_args.push_back(da);
-    CK(cudaMalloc(&dp, prefix.size() * sizeof(long long)));
+    CK(cudaMalloc(&dp, prefix.size() * sizeof(int)));
     e->d_prefix.push_back(dp);
     CK(cudaMemcpy(da, args.data(), args.size() * sizeof(SolveArgs), cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(dp, prefix.data(), prefix.size() * sizeof(long long), cudaMemcpyHostToDevice));
+    CK(cudaMemcpy(dp, prefix.data(), prefix.size() * sizeof(int), cudaMemcpyHostToDevice));
     e->nsub.push_back((int)args.size());
     e->total.push_back(prefix.back());
   }
@@ -2834,7 +2890,7 @@ int ens_enqueue(coral_ensemble* e, double dt) {
   for (int i = 0; i < S; ++i) {
     nl += ens_fan(e, [&](coral_handle* h) { return enqueue_stage_pre(h, i, dt, nullptr); });
     if (e->batched) {
-      launch_subst_multi(e->d_args[i], e->d_prefix[i], e->nsub[i], e->total[i], e->stream);
+      launch_subst_multi(e->d_args[i], e->d_prefix[i], e->nsub[i], e->total[i], e->wide, e->stream);
       ++nl;
     } else {
       nl += ens_fan(e, [&](coral_handle* h) { return enqueue_stage_subst(h, i, dt, nullptr); });

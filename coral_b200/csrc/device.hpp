@@ -238,14 +238,24 @@ struct SolveArgs {
   const int* col_pos;    // [T] class position of a variable column (null: unsplit)
   const unsigned char* colflip_cls;  // [ncls*Tc] colflip in class order
   DevEll Lp;             // L with its columns in class positions (= L when unsplit)
-  // thread-per-block solve (class split): block b = 2 act + class, lane b % 32 of
-  // group b / 32; factors abr[((g Tc + j) ldab + r) 32 + lane], pivots
-  // dpiv[(g Tc + j) 32 + lane], right-hand sides / solutions of the active
-  // systems work2[(g Tc + j) 32 + lane]; inactive systems stay in work
+  // block solve (class split): a unit is one factorisation, shared by the systems
+  // (kx, ky) and (kx, -ky) when the recipe has the ky mirror symmetry; a group is
+  // upw units (16 with the symmetry, else 32) of one class, 32 lanes = the
+  // right-hand sides of its units (mirror symmetry: lanes 16-31 are the -ky
+  // systems).  Group G = class * ngrp + g; packed factors lpack / upack (see
+  // k_pack), pivots dpiv[(G Tc + j) upw + unit], right-hand sides and solutions
+  // work2[(G Tc + j) 32 + lane].
   double2* work2;        // null: warp-per-system layouts
-  int nblk;              // ncls * nact
-  const int* cls_col;    // [ncls*Tc] variable column of a class position, -1 = padding: the
-                         // thread-per-block solve writes its solution straight into out
+  int upw, ngrp;
+  const int* slot;       // [kx*NYA+ky] 32 g + lane of an active system, bit 30: its -ky partner's unit
+  const int* lane_sid;   // [32 ngrp] kx*NYA+ky of a lane's system, -1 = none
+  const unsigned char* row_neg;  // [T] rows negated for the -ky system of a unit
+  const double* lpack;
+  const double* upack;
+  const uint4* finfo;    // [2 Tc] per class and column: its L record (k_pack_info)
+  const uint4* binfo;    // [2 Tc] per class and step of the backward sweep: its U record, variable column
+                         // and signs
+  const int* ptot;       // [4] rows per group of lpack and upack: (class 0, class 1) of each
   // operator-stationary K_std (null tile_win: k_kstd_out): rows in tiles of
   // kTileRows; tile_win[2 tile + .] = (start, width) of the solution columns the
   // tile's rows of L touch; Lw = L with its columns relative to that window
@@ -265,11 +275,8 @@ struct SolveArgs {
   DevGEll NLg;           // NLw in grouped form (valid = 0: none)
   int generic_tiles;     // 1: the tile kernels' run-time forms only (no compiled group layouts)
   int subst_rt;          // 1: the run-time-band substitution kernel even for the compiled band
-  // band entries that are zero in every block are not loaded (FactorArgs::lmask,
-  // umask; null: load all)
-  const unsigned* lmask;
-  const unsigned* umask;
 };
+constexpr int kMirrorBit = 1 << 30;  // SolveArgs::slot
 void launch_solve(const SolveArgs& a, cudaStream_t s);
 // real-scaled factors (unsplit: kl <= 31, kl+ku <= 63; class split: kl <= 15,
 // kl+ku <= 31 per class): right-hand side with the NL assembly fused in,
@@ -280,12 +287,12 @@ void launch_rhs_nl(const SolveArgs& a, const NLArgs& n, cudaStream_t s);
 void launch_subst(const SolveArgs& a, cudaStream_t s);
 void launch_kstd_out(const SolveArgs& a, cudaStream_t s);
 // the substitutions of several systems in one persistent launch (ensembles):
-// d_args[m] the SolveArgs of member m, d_prefix[m] its first block in the
+// d_args[m] the SolveArgs of member m, d_prefix[m] its first group in the
 // concatenated range (d_prefix[nmem] = total); every member must pass
-// subst_multi_supported (thread-per-block layout, band (9, 23), ldab 34)
+// subst_multi_supported (block layout, band (9, 23)); wide: some member's groups
+// have 32 units
 bool subst_multi_supported(const SolveArgs& a);
-void launch_subst_multi(const SolveArgs* d_args, const long long* d_prefix, int nmem, long long total,
-                        cudaStream_t s);
+void launch_subst_multi(const SolveArgs* d_args, const int* d_prefix, int nmem, int total, bool wide, cudaStream_t s);
 
 struct FactorArgs {
   Dims d;
@@ -305,15 +312,19 @@ struct FactorArgs {
   int ncls, Tc;
   const int* cls_row;    // [ncls*Tc] equation row of a class position, -1 = identity padding
   const int* col_pos;    // [T] class position of a variable column
-  int tpb;               // 1: interleaved thread-per-block factor layout (see SolveArgs::work2)
-  int window;            // thread-per-block layout: 1 shared-memory band window, 0 in place in global memory
-  // thread-per-block layout: per class column j, the band rows nonzero in any
-  // block (cmask, bit r = band row r), and derived from it the L rows
-  // (lmask[j], bit i = row kl+ku+1+i of column j) and the U entries of row j
-  // (umask[j], bit i = entry (j, j+1+i)) that are nonzero in any block
-  unsigned long long* cmask;
-  unsigned* lmask;
-  unsigned* umask;
+  // block layout (see SolveArgs::work2; act_list then lists the units' systems,
+  // nact their number): factors abr[((G Tc + j) ldab + r) upw + unit], packed for
+  // the substitution into lpack / upack by k_pack
+  int tpb, upw, ngrp;
+  int window;            // block layout: 1 shared-memory band window, 0 in place in global memory
+  unsigned long long* cmask;  // [2 Tc] per class and column, the band rows nonzero in any unit
+  double* lpack;
+  double* upack;
+  uint4* finfo;
+  uint4* binfo;
+  int* ptot;
+  const int* cls_col;    // [2 Tc] variable column of a class position, -1 = padding
+  const unsigned char* col_neg;  // [T]
 };
 void launch_factor(const FactorArgs& a, cudaStream_t s);
 void launch_factor_real(const FactorArgs& a, cudaStream_t s);

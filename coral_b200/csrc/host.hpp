@@ -166,6 +166,13 @@ struct SystemOps {
   // (variables) of that diagonal scaling and real_scalable is true.
   bool real_scalable = false;
   std::vector<unsigned char> row_flip, col_flip;
+  // Mirror symmetry in ky: when multiplying some equations and some variables by
+  // -1 turns E(kx, ky) into E(kx, -ky) (every entry's power of ky has the parity
+  // of its equation's plus its variable's mark), row_neg[t] / col_neg[t] mark
+  // them and ky_mirror is true: the two systems share one LU factorisation,
+  // exactly (pivot choices compare magnitudes, and signs commute with rounding).
+  bool ky_mirror = false;
+  std::vector<unsigned char> row_neg, col_neg;
   // Independent blocks: when the pattern of M and L (equation rows x variable
   // columns) falls apart into blocks that touch only themselves (Chebyshev
   // parity does this for the plane-layer recipes), the components are gathered

@@ -685,14 +685,15 @@ SystemOps assemble_system(const Geometry& g, const Recipe& r, const CoupledSet& 
     finish_ell(o.NLop, o.T, tr);
     if (o.NLop.groups.empty()) o.NLop.groups.emplace_back(0, 0);
   }
-  // real scaling: parity of (i kx)^a (i ky)^b is a+b; an entry of equation e and
-  // variable v becomes real under the scaling iff r_e = (a+b+s_v) mod 2
-  {
+  // marks of equations and variables such that every piece (e, v) of M and L has
+  // parity(piece) = mark(e) + mark(v) mod 2, spread over the operator's rows and
+  // columns; false when there are none
+  auto two_colour = [&](auto&& parity, std::vector<unsigned char>& row, std::vector<unsigned char>& col) {
     const int nV = o.nV;
     std::vector<int> r_e(nV, -1), s_v(nV, -1);
     std::vector<std::array<int, 3>> edges;  // (e, v, parity)
     for (const auto* pieces : {&s.mass, &s.stif})
-      for (const Piece& p : *pieces) edges.push_back({p.iEqn, p.jVar, (p.kx + p.ky) & 1});
+      for (const Piece& p : *pieces) edges.push_back({p.iEqn, p.jVar, parity(p) & 1});
     bool ok = true;
     // propagate from each unlabelled equation
     for (int start = 0; start < nV && ok; ++start) {
@@ -711,16 +712,20 @@ SystemOps assemble_system(const Geometry& g, const Recipe& r, const CoupledSet& 
     }
     for (int v = 0; v < nV; ++v)
       if (s_v[v] < 0) s_v[v] = 0;
-    o.real_scalable = ok;
-    o.row_flip.assign(o.T, 0);
-    o.col_flip.assign(o.T, 0);
+    row.assign(o.T, 0);
+    col.assign(o.T, 0);
     if (ok) {
       for (int e = 0; e < nV; ++e)
-        for (int rr : o.eq_pos[e]) o.row_flip[rr] = (unsigned char)r_e[e];
+        for (int rr : o.eq_pos[e]) row[rr] = (unsigned char)r_e[e];
       for (int v = 0; v < nV; ++v)
-        for (int c : o.var_pos[v]) o.col_flip[c] = (unsigned char)s_v[v];
+        for (int c : o.var_pos[v]) col[c] = (unsigned char)s_v[v];
     }
-  }
+    return ok;
+  };
+  // real scaling: (i kx)^a (i ky)^b is real or imaginary by the parity of a + b
+  o.real_scalable = two_colour([](const Piece& p) { return p.kx + p.ky; }, o.row_flip, o.col_flip);
+  // ky -> -ky changes its sign by the parity of b
+  o.ky_mirror = two_colour([](const Piece& p) { return p.ky; }, o.row_neg, o.col_neg);
   // stencil rows and square stencils
   o.stencil_rows.resize(o.nV);
   o.sq_stencil.resize(o.nV);

@@ -1611,27 +1611,40 @@ __global__ void __launch_bounds__(kWPBr * 32) k_subst_real(SolveArgs a) {
 
 
 // ------------------------------------------------------------------------------
-// Thread-per-block solve of the independent blocks (class split).  Block
-// b = ncls * act + class is handled by one thread; the 32 blocks of a group lie
-// side by side in memory (abr[((g Tc + j) ldab + r) 32 + lane]), so every factor
-// row, pivot byte and vector entry a warp touches in one step is one contiguous
-// 256 / 32 / 512-byte row.  A thread keeps its band window in its own
-// shared-memory column (slot stride kTpbThreads), where the data-dependent
-// row interchange is a plain indexed access.
+// Block factorisation of the independent blocks (class split).  The block of
+// unit u (one factorisation, of system act_list[u]) and one class is handled by
+// one thread; the upw blocks of a group (one class) lie side by side in memory
+// (abr[((G Tc + j) ldab + r) upw + lane], G = class * ngrp + u / upw), so the
+// accesses of a warp in one step are contiguous rows.
 // ------------------------------------------------------------------------------
 constexpr int kTpbThreads = 128;
 
-// DGBTF2 on one block, in the interleaved layout: the algorithm, pivot choice
-// and update order of k_factor_real.
-// Assembly of block b (system b / ncls, class b % ncls) of M - dt a(0,0) L into
-// its interleaved band storage: zero fill, then every operator entry added in
-// row order (M before L, slots in order).
+// thread b of the block kernels: class, unit, and its column of the group's
+// factors and pivots; false for the padding lanes
+struct TpbBlock {
+  int cls, unit;
+  double* F;
+  unsigned char* P;
+};
+__device__ __forceinline__ bool tpb_block(const FactorArgs& a, int b, TpbBlock& t) {
+  const int G = b / a.upw, lane = b - G * a.upw;
+  if (G >= a.ncls * a.ngrp) return false;
+  t.cls = G / a.ngrp;
+  t.unit = (G - t.cls * a.ngrp) * a.upw + lane;
+  t.F = a.abr + (size_t)G * a.Tc * a.ldab * a.upw + lane;
+  t.P = a.dpiv + (size_t)G * a.Tc * a.upw + lane;
+  return t.unit < a.nact;
+}
+
+// Assembly of one block of M - dt a(0,0) L into its interleaved band storage:
+// zero fill, then every operator entry added in row order (M before L, slots in
+// order).
 // G: the monomial groups the coefficient registers hold (>= the operators' ngroups)
 template <int G = kMaxGroups>
-__device__ void assemble_tpb(const FactorArgs& a, int b) {
-  const int sys = b / a.ncls, cls = b - sys * a.ncls;
-  const int T = a.Tc, kl = a.kl, ku = a.ku, kv = kl + ku, ldab = a.ldab;
-  const int sid = a.act_list[sys];
+__device__ void assemble_tpb(const FactorArgs& a, const TpbBlock& tb) {
+  const int cls = tb.cls;
+  const int T = a.Tc, kl = a.kl, ku = a.ku, kv = kl + ku, ldab = a.ldab, RW = a.upw;
+  const int sid = a.act_list[tb.unit];
   const int kx = sid / a.d.NYA, ky = sid - kx * a.d.NYA;
   double2 cm[G], cl[G];
 #pragma unroll
@@ -1639,8 +1652,8 @@ __device__ void assemble_tpb(const FactorArgs& a, int b) {
     cm[g] = (g < a.M.ngroups) ? cmul(ipow(a.kx[kx], a.M.gkx[g]), ipow(a.ky[ky], a.M.gky[g])) : zero2();
     cl[g] = (g < a.L.ngroups) ? cmul(ipow(a.kx[kx], a.L.gkx[g]), ipow(a.ky[ky], a.L.gky[g])) : zero2();
   }
-  double* F = a.abr + (size_t)(b >> 5) * T * ldab * 32 + (b & 31);
-  auto at = [&](int j, int r) -> double& { return F[((size_t)j * ldab + r) * 32]; };
+  double* F = tb.F;
+  auto at = [&](int j, int r) -> double& { return F[((size_t)j * ldab + r) * RW]; };
   for (int j = 0; j < T; ++j)
     for (int r = 0; r < ldab; ++r) at(j, r) = 0.0;
   for (int i = 0; i < T; ++i) {
@@ -1672,19 +1685,22 @@ __device__ void assemble_tpb(const FactorArgs& a, int b) {
 
 template <int G>
 __global__ void __launch_bounds__(kTpbThreads) k_assemble_tpb(FactorArgs a) {
-  const int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b < a.ncls * a.nact) assemble_tpb<G>(a, b);
+  TpbBlock tb;
+  if (tpb_block(a, blockIdx.x * blockDim.x + threadIdx.x, tb)) assemble_tpb<G>(a, tb);
 }
 
+// DGBTF2 on one block in place in global memory: the algorithm, pivot choice and
+// update order of k_factor_real.
+
 __global__ void __launch_bounds__(kTpbThreads) k_factor_tpb(FactorArgs a) {
-  const int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= a.ncls * a.nact) return;
-  assemble_tpb(a, b);
-  const int sys = b / a.ncls;
+  TpbBlock tb;
+  if (!tpb_block(a, blockIdx.x * blockDim.x + threadIdx.x, tb)) return;
+  assemble_tpb(a, tb);
+  const int sys = tb.unit, RW = a.upw;
   const int T = a.Tc, kl = a.kl, ku = a.ku, kv = kl + ku, ldab = a.ldab;
-  double* F = a.abr + (size_t)(b >> 5) * T * ldab * 32 + (b & 31);
-  auto at = [&](int j, int r) -> double& { return F[((size_t)j * ldab + r) * 32]; };
-  unsigned char* P = a.dpiv + (size_t)(b >> 5) * T * 32 + (b & 31);
+  double* F = tb.F;
+  auto at = [&](int j, int r) -> double& { return F[((size_t)j * ldab + r) * RW]; };
+  unsigned char* P = tb.P;
   int ju = 0, info = 0;
   for (int j = 0; j < T; ++j) {
     const int km = min(kl, T - 1 - j);
@@ -1694,7 +1710,7 @@ __global__ void __launch_bounds__(kTpbThreads) k_factor_tpb(FactorArgs a) {
       const double m2 = fabs(at(j, kv + i));
       if (m2 > mag) { mag = m2; jp = i; }  // first maximum
     }
-    P[(size_t)j * 32] = (unsigned char)jp;
+    P[(size_t)j * RW] = (unsigned char)jp;
     if (at(j, kv + jp) == 0.0) {
       if (info == 0) info = j + 1;
       continue;
@@ -1743,25 +1759,25 @@ __device__ __forceinline__ void cp_async8(void* smem, const void* gmem) {
 __global__ void __launch_bounds__(32) k_factor_win(FactorArgs a) {
   extern __shared__ double fwin[];
   const int NT = blockDim.x;
-  const int b = blockIdx.x * NT + threadIdx.x;
-  if (b >= a.ncls * a.nact) return;  // no barriers below
-  const int sys = b / a.ncls;
+  TpbBlock tb;
+  if (!tpb_block(a, blockIdx.x * NT + threadIdx.x, tb)) return;  // no barriers below
+  const int sys = tb.unit, RW = a.upw;
   const int T = a.Tc, kl = a.kl, ku = a.ku, kv = kl + ku, ldab = a.ldab, W = kl + ku + 1, W1 = W + 1;
-  double* F = a.abr + (size_t)(b >> 5) * T * ldab * 32 + (b & 31);
+  double* F = tb.F;
   double* wz = fwin + threadIdx.x;
   int j0 = 0, s0 = 0;  // the window's first column and its slot
   auto slot = [&](int c) { const int q = s0 + (c - j0); return q >= W1 ? q - W1 : q; };
   auto at = [&](int c, int r) -> double& { return wz[(slot(c) * ldab + r) * NT]; };
   auto fetch = [&](int c, int sl) {  // column c of the block into slot sl
     if (c < T) {
-      const double* src = F + (size_t)c * ldab * 32;
+      const double* src = F + (size_t)c * ldab * RW;
       double* dst = wz + (size_t)sl * ldab * NT;
-      for (int r = 0; r < ldab; ++r) cp_async8(dst + r * NT, src + (size_t)r * 32);
+      for (int r = 0; r < ldab; ++r) cp_async8(dst + r * NT, src + (size_t)r * RW);
     }
   };
   for (int c = 0; c < W; ++c) fetch(c, c);
   cp_async_commit();
-  unsigned char* P = a.dpiv + (size_t)(b >> 5) * T * 32 + (b & 31);
+  unsigned char* P = tb.P;
   int ju = 0, info = 0;
   for (int j = 0; j < T; ++j) {
     j0 = j;
@@ -1775,7 +1791,7 @@ __global__ void __launch_bounds__(32) k_factor_win(FactorArgs a) {
       const double m2 = fabs(at(j, kv + i));
       if (m2 > mag) { mag = m2; jp = i; }  // first maximum
     }
-    P[(size_t)j * 32] = (unsigned char)jp;
+    P[(size_t)j * RW] = (unsigned char)jp;
     if (at(j, kv + jp) == 0.0) {
       if (info == 0) info = j + 1;
     } else {
@@ -1815,295 +1831,452 @@ __global__ void __launch_bounds__(32) k_factor_win(FactorArgs a) {
     }
     // column j is final
     const double* cw = wz + (size_t)s0 * ldab * NT;
-    double* dst = F + (size_t)j * ldab * 32;
-    for (int q = 0; q < ldab; ++q) dst[(size_t)q * 32] = cw[q * NT];
+    double* dst = F + (size_t)j * ldab * RW;
+    for (int q = 0; q < ldab; ++q) dst[(size_t)q * RW] = cw[q * NT];
     s0 = (s0 + 1 == W1) ? 0 : s0 + 1;
   }
   cp_async_wait<0>();
   if (info) atomicMax(a.info + sys, info);
 }
 
-// Band rows that are nonzero in any block, per class column: one warp per
-// (group, column) tests the 32 blocks of its group row by row (lanes beyond
-// the last block count as zero).
+// Band rows that are nonzero in any unit, per class and column: one warp per
+// (group, column) tests the units of its group row by row (padding lanes count
+// as zero).
 __global__ void __launch_bounds__(256) k_mask_cols(FactorArgs a) {
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int g = blockIdx.x, j = blockIdx.y * 8 + w;
+  const int G = blockIdx.x, j = blockIdx.y * 8 + w;
   const int T = a.Tc, ldab = a.ldab;
   if (j >= T) return;
-  const bool ok = g * 32 + lane < a.ncls * a.nact;
-  const double* F = a.abr + ((size_t)g * T + j) * ldab * 32 + lane;
+  const int cls = G / a.ngrp, u0 = (G - cls * a.ngrp) * a.upw;
+  const bool ok = lane < a.upw && u0 + lane < a.nact;
+  const double* F = a.abr + ((size_t)G * T + j) * ldab * a.upw + (ok ? lane : 0);
   unsigned long long bits = 0;
   for (int r = 0; r < ldab; ++r) {
-    const double v = ok ? F[(size_t)r * 32] : 0.0;
+    const double v = ok ? F[(size_t)r * a.upw] : 0.0;
     if (__any_sync(0xffffffffu, v != 0.0)) bits |= 1ull << r;
   }
-  if (lane == 0 && bits) atomicOr(a.cmask + j, bits);
+  if (lane == 0 && bits) atomicOr(a.cmask + (size_t)cls * T + j, bits);
 }
-// lmask / umask from cmask (see FactorArgs)
-__global__ void k_mask_rows(FactorArgs a) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
+// The records of the substitution from cmask, one warp per class.  A factor row
+// is upw doubles (one entry of every unit of a group).  Forward: column j's
+// record in lpack is its L rows i (band row kl+ku+1+i) that are nonzero in some
+// unit.  Backward: step k handles row j = Tc-1-k; its record in upack is the
+// reciprocal diagonal (row 0) and the entries (j, j+i) (row i) that are nonzero
+// in some unit.  Rows in increasing i.
+//   finfo[k] = first row, mask of the rows held
+//   binfo[k] = first row, mask of the rows held, variable column (-1 = padding),
+//              bit 0 colflip, bit 1 col_neg
+// ptot: rows per group.
+__global__ void __launch_bounds__(32) k_pack_info(FactorArgs a) {
+  const int lane = threadIdx.x, cls = blockIdx.x;
   const int T = a.Tc, kl = a.kl, kv = a.kl + a.ku;
-  if (j >= T) return;
-  a.lmask[j] = (unsigned)((a.cmask[j] >> (kv + 1)) & ((1ull << kl) - 1));
-  unsigned u = 0;
-  for (int i = 0; i < kv; ++i)
-    if (j + 1 + i < T && ((a.cmask[j + 1 + i] >> (kv - 1 - i)) & 1ull)) u |= 1u << i;
-  a.umask[j] = u;
+  const unsigned long long* cm = a.cmask + (size_t)cls * T;
+  int base[2] = {0, 0};
+  for (int k0 = 0; k0 < T; k0 += 32) {
+    const int k = k0 + lane;
+    unsigned lm = 0, um = 0;
+    if (k < T) {
+      lm = (unsigned)((cm[k] >> (kv + 1)) & ((1ull << kl) - 1));
+      const int j = T - 1 - k;
+      um = 1u;
+      for (int i = 1; i <= kv; ++i)
+        if (j + i < T && ((cm[j + i] >> (kv - i)) & 1ull)) um |= 1u << i;
+    }
+    const int n[2] = {__popc(lm), __popc(um)};
+    int off[2];
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      int inc = n[q];
+      for (int o = 1; o < 32; o <<= 1) {
+        const int up = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += up;
+      }
+      off[q] = base[q] + inc - n[q];
+      base[q] += __shfl_sync(0xffffffffu, inc, 31);
+    }
+    if (k < T) {
+      const size_t at = (size_t)cls * T + k;
+      a.finfo[at] = make_uint4((unsigned)off[0], lm, 0u, 0u);
+      const int t = a.cls_col[(size_t)cls * T + T - 1 - k];
+      const unsigned fl = t >= 0 ? (a.colflip[t] ? 1u : 0u) | (a.col_neg[t] ? 2u : 0u) : 0u;
+      a.binfo[at] = make_uint4((unsigned)off[1], um, (unsigned)t, fl);
+    }
+  }
+  if (lane == 0) {
+    a.ptot[cls] = base[0];
+    a.ptot[2 + cls] = base[1];
+  }
+}
+// first row of group G's records in lpack (q = 0) or upack (q = 1)
+__device__ __forceinline__ size_t pack_base(const int* ptot, int q, int cls, int g, int ngrp) {
+  const int t0 = ptot[2 * q], t1 = ptot[2 * q + 1];
+  return cls == 0 ? (size_t)g * t0 : (size_t)ngrp * t0 + (size_t)g * t1;
+}
+// The band factors copied into the records: one warp per (group, column).  The
+// substitution then reads two linear streams that hold only what it needs.
+__global__ void __launch_bounds__(256) k_pack(FactorArgs a) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int G = blockIdx.x, k = blockIdx.y * 8 + w;
+  const int T = a.Tc, kv = a.kl + a.ku, ldab = a.ldab, RW = a.upw;
+  if (k >= T) return;
+  const int cls = G / a.ngrp, g = G - cls * a.ngrp;
+  const double* F = a.abr + (size_t)G * T * ldab * RW;
+  const int half = lane / RW, ln = lane - half * RW, per = 32 / RW;  // rows a warp copies at a time
+  {
+    const uint4 fi = a.finfo[(size_t)cls * T + k];
+    double* dst = a.lpack + (pack_base(a.ptot, 0, cls, g, a.ngrp) + fi.x) * RW;
+    const int n = __popc(fi.y);
+    for (int r = half; r < n; r += per) {
+      const int i = __fns(fi.y, 0, r + 1);  // the (r + 1)-th set bit
+      dst[(size_t)r * RW + ln] = F[((size_t)k * ldab + kv + 1 + i) * RW + ln];
+    }
+  }
+  {
+    const uint4 bi = a.binfo[(size_t)cls * T + k];
+    double* dst = a.upack + (pack_base(a.ptot, 1, cls, g, a.ngrp) + bi.x) * RW;
+    const int j = T - 1 - k, n = __popc(bi.y);
+    for (int r = half; r < n; r += per) {
+      const int i = __fns(bi.y, 0, r + 1);
+      dst[(size_t)r * RW + ln] = F[((size_t)(j + i) * ldab + kv - i) * RW + ln];
+    }
+  }
 }
 
-// Forward (P, L: the column sweep with the row interchanges interleaved, as the
-// reference's band solve) then backward (U, row form: each x_j subtracts the
-// known x_{j+i} in decreasing column order, the order in which the column sweep
-// reaches it) for one block.  The band is compile-time (kl = KL, kl + ku = KV,
-// column stride LD = ldab), so every factor offset is an immediate from one
-// per-column pointer; each step's factor values are loaded one step ahead.
-// Band entries outside the matrix are stored zeros, so the forward sweep runs
-// unpredicated (it only touches dead window slots near the end); the backward
-// rows within KV of the last column take the guarded loop.
-// The substitution of block b of the system described by a; win is this
-// thread's band-window column in shared memory (slot stride kTpbThreads).
-template <int KL, int KV, int LD>
-__device__ __forceinline__ void subst_tpb_block(const SolveArgs& a, int b, double2* win) {
-  constexpr int W1 = (KL + 2 <= 16) ? 16 : 32;  // power of 2 >= KL + 2
-  constexpr int W2 = KV + 1;
-  constexpr int S = kTpbThreads;                // slot stride
-  constexpr size_t CS = (size_t)LD * 32;        // column stride (doubles)
-  const int T = a.Tc;
-  const int cls = b % a.ncls;
-  const size_t gb = (size_t)(b >> 5) * T;
-  const double* F = a.abr + gb * CS + (b & 31);
-  const unsigned char* P = a.dpiv + gb * 32 + (b & 31);
-  double2* X = a.work2 + gb * 32 + (b & 31);
-  const unsigned char* cflip = a.colflip_cls + (size_t)cls * T;
-  const int* ccol = a.cls_col + (size_t)cls * T;
-  double2* out = a.out + (size_t)a.act_list[b / a.ncls] * a.T;  // this system's stage output
-  bool bad = false;
-  // ---- forward: positions j..j+KL in slots p mod W1 ----
-  for (int p = 0; p <= KL && p < T; ++p) win[(p & (W1 - 1)) * S] = X[(size_t)p * 32];
-  // L rows / U entries that are zero in every block are not loaded
-  const unsigned* lmask = a.lmask;
-  const unsigned* umask = a.umask;
-  if (T > 1) {
-    double lv[KL], lvn[KL];
-    int jpn = P[0];
-    double2 incn = (KL + 1 < T) ? X[(size_t)(KL + 1) * 32] : zero2();
-    {
-      const unsigned lm = lmask ? lmask[0] : ~0u;
+// ------------------------------------------------------------------------------
+// Band substitutions of one group by one warp: forward (P, L: the column sweep
+// with the row interchanges interleaved, as the reference's band solve) then
+// backward (U, row form: each x_j subtracts the known x_{j+i} in decreasing
+// column order, the order in which the column sweep reaches it); the solution,
+// scaled back, goes straight into the stage output.
+//
+// What bounds it: the factor and vector streams on large grids, the chain of 2 Tc
+// dependent column steps on small ones.  So (a) the systems (kx, ky) and
+// (kx, -ky) share one factorisation where the recipe's mirror symmetry allows: 16
+// units a warp, two right-hand sides each, half the factor bytes; (b) the factors
+// come as linear streams of the entries that are nonzero in some unit (k_pack);
+// (c) both streams, the right-hand sides and the intermediate vector are copied
+// with cp.async into a ring in shared memory DF (forward) or DB (backward)
+// columns ahead, so that a column step waits for shared memory only.  Against
+// one thread per system that loads its factors one column ahead, no-slip
+// convection, per launch: 384^2 x 192 3.83 -> 2.42 ms (14.1 GB, 5.8 TB/s),
+// 128^2 x 192 1.26 -> 0.39 ms, 64^2 x 48 0.318 -> 0.099 ms; without the symmetry
+// (rotating, 192^2 x 96) 0.72 -> 0.49 ms.
+//
+// The window of the vector (rows j .. j+KL, x_{j+1} .. x_{j+KV}) is in registers:
+// U column steps are unrolled, so that every row has a fixed register, and the
+// window moves by U rows after them; the row interchange is a chain of selects.
+// (With the window in shared memory the kernel was bound by that memory's
+// accesses, 75% of the LSU's peak at 256^2 x 96, 1.76 ms per step.)  The ring
+// holds a record's rows at fixed places (holes zero-filled by the copies), the
+// rows that most records hold are handled without a test, a step's factors are
+// read from the ring one step ahead, and the record descriptions come in blocks of
+// 32, one per lane.
+// ------------------------------------------------------------------------------
+template <int KL, int KV, int UPW>
+struct SubstShape {
+  static constexpr int DF = 6, DB = UPW == 16 ? 5 : 4;        // columns copied ahead
+  static constexpr int kLBytes = KL * UPW * 8;
+  static constexpr int kFSlot = kLBytes + UPW + 512;          // L rows, pivot bytes, row j + KL of the vector
+  static constexpr int kUBytes = (KV + 1) * UPW * 8;
+  static constexpr int kBSlot = kUBytes + 512;                // U rows, row j of the vector
+  static constexpr int kRingF = (DF + 1) * kFSlot, kRingB = (DB + 1) * kBSlot;
+  static constexpr int kBytes = kRingF > kRingB ? kRingF : kRingB;
+  static_assert(kFSlot % 16 == 0 && kBSlot % 16 == 0, "16-byte copies");
+};
+__device__ __forceinline__ void cp_async16s(unsigned sa, const void* gmem) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(sa), "l"(gmem) : "memory");
+}
+// One warp copies a record (the rows of mask m, contiguous at src) to rows i =
+// 0 .. ROWS-1 at dst, zeros where m has no bit.  Rows from HARD on are left alone
+// where no row of their group of kRowGroup is held.
+constexpr int kRowGroup = 4;
+template <int ROWS, int HARD, int UPW>
+__device__ __forceinline__ void record_copy(unsigned dst, const char* src, unsigned m, int lane) {
+  constexpr int GPR = UPW / 2, RPC = 32 / GPR;  // 16-byte granules per row, rows per 512-byte piece
+  const int il = lane / GPR, w = (lane % GPR) * 16;
 #pragma unroll
-      for (int i = 0; i < KL; ++i) lvn[i] = ((lm >> i) & 1u) ? F[(KV + 1 + i) * 32] : 0.0;
-    }
-    for (int j = 0; j < T - 1; ++j) {
-#pragma unroll
-      for (int i = 0; i < KL; ++i) lv[i] = lvn[i];
-      const int jp = jpn;
-      const double2 inc = incn;
-      if (j + 1 < T - 1) {  // next column's multipliers, pivot and incoming entry
-        const double* Fn = F + (size_t)(j + 1) * CS;
-        const unsigned lm = lmask ? lmask[j + 1] : ~0u;
-#pragma unroll
-        for (int i = 0; i < KL; ++i) lvn[i] = ((lm >> i) & 1u) ? Fn[(KV + 1 + i) * 32] : 0.0;
-        jpn = P[(size_t)(j + 1) * 32];
-        incn = (j + KL + 2 < T) ? X[(size_t)(j + KL + 2) * 32] : zero2();
-      }
-      const int s0 = j & (W1 - 1);
-      const int sp = (j + jp) & (W1 - 1);
-      const double2 bj = win[sp * S];
-      if (jp) win[sp * S] = win[s0 * S];
-#pragma unroll
-      for (int i = 0; i < KL; ++i) {
-        const int sl = (s0 + 1 + i) & (W1 - 1);
-        double2 w = win[sl * S];
-        w.x -= lv[i] * bj.x;
-        w.y -= lv[i] * bj.y;
-        win[sl * S] = w;
-      }
-      X[(size_t)j * 32] = bj;
-      if (j + KL + 1 < T) win[((j + KL + 1) & (W1 - 1)) * S] = inc;
+  for (int q = 0; q * RPC < ROWS; ++q) {
+    const int i = q * RPC + il;
+    if (q * RPC < HARD || ((m >> (q * RPC / kRowGroup * kRowGroup)) & ((1u << kRowGroup) - 1))) {
+      const unsigned sa = dst + q * 512 + lane * 16;
+      const char* p = src + __popc(m & ((1u << i) - 1)) * (UPW * 8) + w;
+      const int n = (m >> i) & 1u ? 16 : 0;
+      if (i < ROWS) asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(sa), "l"(p), "r"(n) : "memory");
     }
   }
-  if (T > 0) X[(size_t)(T - 1) * 32] = win[((T - 1) & (W1 - 1)) * S];
-  // ---- backward: x_{j+1}..x_{j+KV} in slots p mod W2 ----
-  int sj = (T - 1) % W2;  // slot of position j
-  int j = T - 1;
-  for (; j >= 0 && j + KV >= T; --j) {  // rows within KV of the end
-    const double* Fj = F + (size_t)j * CS;
-    double2 acc = X[(size_t)j * 32];
-    for (int i = T - 2 - j; i >= 0; --i) {
-      int sl = sj + 1 + i;
-      if (sl >= W2) sl -= W2;
-      const double u = Fj[((1 + i) * LD + KV - 1 - i) * 32];
-      const double2 xv = win[sl * S];
-      acc.x -= u * xv.x;
-      acc.y -= u * xv.y;
-    }
-    const double dinv = Fj[KV * 32];  // U's diagonal is stored as its reciprocal
-    const double2 xj = make_double2(acc.x * dinv, acc.y * dinv);
-    win[sj * S] = xj;
-    {  // the solution, scaled back, straight into the stage output (original order)
-      const int t = ccol[j];
-      if (t >= 0) {
-        const double2 xo = flip_col(xj, cflip[j]);
-        bad |= !(isfinite(xo.x) && isfinite(xo.y));
-        out[t] = xo;
-      }
-    }
-    sj = (sj == 0) ? W2 - 1 : sj - 1;
+}
+// Descriptions of consecutive records k = 0 .. n-1, one per lane for a block of 32
+// and the next block: rec(k) for k in the current or the next block, col(k) for k
+// in the current one; next(k) after record k.
+struct RecordBlock {
+  const uint4* src;
+  int n, base, lane;
+  uint4 cur, nxt;
+  __device__ __forceinline__ uint4 load(int k) const {
+    return k < n ? __ldg(src + k) : make_uint4(0u, 0u, 0u, 0u);
   }
-  if (j >= 0) {
-    double u[KV], un[KV];
-    double dinv, dinvn;
-    double2 yn;
-    {
-      const double* Fj = F + (size_t)j * CS;
-      const unsigned um = umask ? umask[j] : ~0u;
-#pragma unroll
-      for (int i = 0; i < KV; ++i) un[i] = ((um >> i) & 1u) ? Fj[((1 + i) * LD + KV - 1 - i) * 32] : 0.0;
-      dinvn = Fj[KV * 32];
-      yn = X[(size_t)j * 32];
+  __device__ __forceinline__ RecordBlock(const uint4* s, int count, int ln) : src(s), n(count), base(0), lane(ln) {
+    cur = load(lane);
+    nxt = load(32 + lane);
+  }
+  __device__ __forceinline__ uint2 rec(int k) const {  // first row, mask
+    const int i = k - base;
+    const unsigned a = i < 32 ? cur.x : nxt.x, b = i < 32 ? cur.y : nxt.y;
+    return make_uint2(__shfl_sync(0xffffffffu, a, i & 31), __shfl_sync(0xffffffffu, b, i & 31));
+  }
+  __device__ __forceinline__ uint2 col(int k) const {  // variable column, signs
+    return make_uint2(__shfl_sync(0xffffffffu, cur.z, k & 31), __shfl_sync(0xffffffffu, cur.w, k & 31));
+  }
+  __device__ __forceinline__ void next(int k) {
+    if ((k & 31) == 31) {
+      base += 32;
+      cur = nxt;
+      nxt = load(base + 32 + lane);
     }
-    for (; j >= 0; --j) {
-#pragma unroll
-      for (int i = 0; i < KV; ++i) u[i] = un[i];
-      dinv = dinvn;
-      double2 acc = yn;
-      if (j > 0) {  // next row (j - 1)
-        const double* Fn = F + (size_t)(j - 1) * CS;
-        const unsigned um = umask ? umask[j - 1] : ~0u;
-#pragma unroll
-        for (int i = 0; i < KV; ++i) un[i] = ((um >> i) & 1u) ? Fn[((1 + i) * LD + KV - 1 - i) * 32] : 0.0;
-        dinvn = Fn[KV * 32];
-        yn = X[(size_t)(j - 1) * 32];
+  }
+};
+
+// b = 2 g + class: the two classes of a group's systems run side by side, so that
+// their interleaved entries of the stage output meet in L2 (class after class:
+// 3.24 instead of 2.42 ms at 384^2 x 192)
+template <int KL, int KV, int UPW>
+__device__ __forceinline__ void subst_group(const SolveArgs& a, int b, unsigned char* ring) {
+  using S = SubstShape<KL, KV, UPW>;
+  constexpr int DF = S::DF, DB = S::DB;
+  constexpr int RB = UPW * 8;  // bytes of a factor row
+  const int lane = threadIdx.x & 31, unit = lane & (UPW - 1);
+  const int T = a.Tc, cls = b & 1, g = b >> 1, G = cls * a.ngrp + g;
+  const int sid = a.lane_sid[g * 32 + lane];
+  const unsigned ring_s = (unsigned)__cvta_generic_to_shared(ring);
+  double2* X = a.work2 + (size_t)G * T * 32 + lane;
+  // ---- forward: rows j .. j+KL at r[s .. s+KL] in step s of the unrolled ones ----
+  {
+    constexpr int U = 4;
+    constexpr int NA = KL < 6 ? KL : 6;       // L rows handled without a test
+    const char* L = reinterpret_cast<const char*>(a.lpack + pack_base(a.ptot, 0, cls, g, a.ngrp) * UPW);
+    const unsigned char* P = a.dpiv + (size_t)G * T * UPW;
+    const int nc = T - 1;  // columns
+    RecordBlock info(a.finfo + (size_t)cls * T, nc, lane);
+    auto issue = [&](int c, int slot, uint2 rec) {  // column c and row c + KL
+      const unsigned dst = ring_s + slot * S::kFSlot;
+      if (c < nc) {
+        record_copy<KL, KL, UPW>(dst, L + (size_t)rec.x * RB, rec.y, lane);
+        if (lane < UPW / 16) cp_async16s(dst + S::kLBytes + lane * 16, P + (size_t)c * UPW + lane * 16);
+        if (c + KL < T) cp_async16s(dst + S::kLBytes + UPW + lane * 16, X + (size_t)(c + KL) * 32);
       }
+    };
 #pragma unroll
-      for (int i = KV - 1; i >= 0; --i) {
-        int sl = sj + 1 + i;
-        if (sl >= W2) sl -= W2;
-        const double2 xv = win[sl * S];
-        acc.x -= u[i] * xv.x;
-        acc.y -= u[i] * xv.y;
-      }
-      const double2 xj = make_double2(acc.x * dinv, acc.y * dinv);
-      win[sj * S] = xj;
-      {  // the solution, scaled back, straight into the stage output (original order)
-        const int t = ccol[j];
-        if (t >= 0) {
-          const double2 xo = flip_col(xj, cflip[j]);
-          bad |= !(isfinite(xo.x) && isfinite(xo.y));
-          out[t] = xo;
+    for (int c = 0; c < DF; ++c) {
+      issue(c, c, info.rec(c));
+      cp_async_commit();
+    }
+    uint2 recn = info.rec(DF);
+    double2 r[KL + U + 1];
+#pragma unroll
+    for (int p = 0; p < KL; ++p) r[p] = p < T ? X[(size_t)p * 32] : zero2();
+    int sw = DF, sr = 0;  // ring slots of columns j + DF and j
+    // a column's pivot, L rows and incoming row, read one step ahead (of a column
+    // past the last: stale, unused)
+    int jp;
+    double l[KL];
+    double2 rin;
+    auto read = [&](int slot, int& piv, double (&lv)[KL], double2& row) {
+      const unsigned char* b = ring + slot * S::kFSlot;
+      piv = b[S::kLBytes + unit];
+#pragma unroll
+      for (int i = 0; i < KL; ++i) lv[i] = reinterpret_cast<const double*>(b)[i * UPW + unit];
+      row = *reinterpret_cast<const double2*>(b + S::kLBytes + UPW + lane * 16);
+    };
+    cp_async_wait<DF - 1>();
+    __syncwarp();
+    read(0, jp, l, rin);
+    for (int j0 = 0; j0 < nc; j0 += U) {
+#pragma unroll
+      for (int s = 0; s < U; ++s) {
+        const int j = j0 + s;
+        if (j < nc) {
+          const unsigned m = info.rec(j).y;
+          cp_async_wait<DF - 2>();  // column j + 1's record is in
+          __syncwarp();             // for every lane; and every lane is done with column j - 1's slot
+          issue(j + DF, sw, recn);
+          cp_async_commit();
+          recn = info.rec(j + DF + 1);
+          int jpn;
+          double ln[KL];
+          double2 rinn;
+          sr = sr == DF ? 0 : sr + 1;
+          sw = sw == DF ? 0 : sw + 1;
+          read(sr, jpn, ln, rinn);
+          r[s + KL] = rin;
+          // row j + jp comes up, row j goes down
+          double2 bj = r[s];
+          const double2 x0 = r[s];
+#pragma unroll
+          for (int i = 1; i <= NA; ++i)
+            if (jp == i) {
+              bj = r[s + i];
+              r[s + i] = x0;
+            }
+          const bool far = KL > NA && ((m >> NA) || __any_sync(0xffffffffu, jp > NA));
+          if (far) {
+#pragma unroll
+            for (int i = NA + 1; i <= KL; ++i)
+              if (jp == i) {
+                bj = r[s + i];
+                r[s + i] = x0;
+              }
+          }
+#pragma unroll
+          for (int i = 0; i < NA; ++i) {
+            r[s + 1 + i].x -= l[i] * bj.x;
+            r[s + 1 + i].y -= l[i] * bj.y;
+          }
+          if (far) {
+#pragma unroll
+            for (int i = NA; i < KL; ++i) {
+              r[s + 1 + i].x -= l[i] * bj.x;
+              r[s + 1 + i].y -= l[i] * bj.y;
+            }
+          }
+          X[(size_t)j * 32] = bj;
+          jp = jpn;
+          rin = rinn;
+#pragma unroll
+          for (int i = 0; i < KL; ++i) l[i] = ln[i];
+          info.next(j);
+          if (j == nc - 1) X[(size_t)nc * 32] = r[s + 1];
         }
       }
-      sj = (sj == 0) ? W2 - 1 : sj - 1;
+#pragma unroll
+      for (int p = 0; p < KL; ++p) r[p] = r[p + U];
     }
+    cp_async_wait<0>();
+    __threadfence();  // the copies below read the intermediate vector back
+    __syncwarp();
   }
-  // non-finite check (no warp-collective operation: lanes of a partial warp returned early)
-  if (bad) atomicOr(a.flags, 1u);
-}
-
-template <int KL, int KV, int LD>
-__global__ void __launch_bounds__(kTpbThreads) k_subst_tpb(SolveArgs a) {
-  extern __shared__ double2 swin[];
-  const int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= a.nblk) return;  // no warp-collective operations below
-  subst_tpb_block<KL, KV, LD>(a, b, swin + threadIdx.x);
-}
-
-// The substitutions of many systems (the members of an ensemble) in one
-// persistent launch: thread slots walk the concatenated block range of all
-// members (member m owns blocks [prefix[m], prefix[m+1])) with a grid stride;
-// each block runs exactly the arithmetic of k_subst_tpb.
-template <int KL, int KV, int LD>
-__global__ void __launch_bounds__(kTpbThreads) k_subst_tpb_multi(const SolveArgs* args, const long long* prefix,
-                                                                 int nmem, long long total) {
-  extern __shared__ double2 swin[];
-  for (long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x; g < total;
-       g += (long long)gridDim.x * blockDim.x) {
-    int lo = 0, hi = nmem - 1;  // member m with prefix[m] <= g < prefix[m+1]
-    while (lo < hi) {
-      const int mid = (lo + hi + 1) >> 1;
-      if (prefix[mid] <= g) lo = mid;
-      else hi = mid - 1;
+  // ---- backward: x_{j+i} at r[U-1-s+i] in step s of the unrolled ones ----
+  {
+    constexpr int U = KV > 24 ? 2 : 4;
+    constexpr int NA = 12;   // U rows handled without a test (row 0 the diagonal)
+    constexpr int CB = kRowGroup;
+    static_assert(NA % CB == 0 && NA <= KV, "groups");
+    const char* Up = reinterpret_cast<const char*>(a.upack + pack_base(a.ptot, 1, cls, g, a.ngrp) * UPW);
+    double2* out = a.out + (size_t)(sid >= 0 ? sid : 0) * a.T;
+    bool bad = false;
+    RecordBlock info(a.binfo + (size_t)cls * T, T, lane);
+    auto issue = [&](int k, int slot, uint2 rec) {
+      if (k < T) {
+        const unsigned dst = ring_s + slot * S::kBSlot;
+        record_copy<KV + 1, NA, UPW>(dst, Up + (size_t)rec.x * RB, rec.y, lane);
+        cp_async16s(dst + S::kUBytes + lane * 16, X + (size_t)(T - 1 - k) * 32);
+      }
+    };
+#pragma unroll
+    for (int c = 0; c < DB; ++c) {
+      issue(c, c, info.rec(c));
+      cp_async_commit();
     }
-    subst_tpb_block<KL, KV, LD>(args[lo], (int)(g - prefix[lo]), swin + threadIdx.x);
+    uint2 recn = info.rec(DB);
+    double2 r[KV + U];
+#pragma unroll
+    for (int p = 0; p < KV + U; ++p) r[p] = zero2();
+    int sw = DB, sr = 0;
+    double u[NA];
+    double2 y;
+    auto read = [&](int slot, double (&uv)[NA], double2& row) {
+      const unsigned char* b = ring + slot * S::kBSlot;
+      row = *reinterpret_cast<const double2*>(b + S::kUBytes + lane * 16);
+#pragma unroll
+      for (int i = 0; i < NA; ++i) uv[i] = reinterpret_cast<const double*>(b)[i * UPW + unit];
+    };
+    cp_async_wait<DB - 1>();
+    __syncwarp();
+    read(0, u, y);
+    for (int k0 = 0; k0 < T; k0 += U) {
+#pragma unroll
+      for (int s = 0; s < U; ++s) {
+        const int k = k0 + s;
+        if (k < T) {
+          const unsigned m = info.rec(k).y;
+          const uint2 col = info.col(k);
+          cp_async_wait<DB - 2>();
+          __syncwarp();
+          issue(k + DB, sw, recn);
+          cp_async_commit();
+          recn = info.rec(k + DB + 1);
+          const double* slot = reinterpret_cast<const double*>(ring + sr * S::kBSlot) + unit;
+          sr = sr == DB ? 0 : sr + 1;
+          sw = sw == DB ? 0 : sw + 1;
+          double un[NA];
+          double2 yn;
+          read(sr, un, yn);
+          // (one sum in the reference's order: the operators' conditioning turns
+          // another order's rounding into 1e-9 of the pressure)
+          double2 acc = y;
+          if (m >> NA) {
+#pragma unroll
+            for (int i0 = (KV - NA) / CB * CB + NA; i0 >= NA; i0 -= CB) {
+              if ((m >> i0) & ((1u << CB) - 1)) {
+#pragma unroll
+                for (int i = i0 + CB - 1; i >= i0; --i)
+                  if (i <= KV) {
+                    const double ui = slot[i * UPW];
+                    acc.x -= ui * r[U - 1 - s + i].x;
+                    acc.y -= ui * r[U - 1 - s + i].y;
+                  }
+              }
+            }
+          }
+#pragma unroll
+          for (int i = NA - 1; i >= 1; --i) {
+            acc.x -= u[i] * r[U - 1 - s + i].x;
+            acc.y -= u[i] * r[U - 1 - s + i].y;
+          }
+          const double2 xj = make_double2(acc.x * u[0], acc.y * u[0]);  // the diagonal is stored as its reciprocal
+          r[U - 1 - s] = xj;
+          const int t = (int)col.x;
+          if (t >= 0 && sid >= 0) {
+            double2 xo = flip_col(xj, col.y & 1u);
+            if (UPW == 16 && lane >= 16 && (col.y & 2u)) xo = make_double2(-xo.x, -xo.y);
+            bad |= !(isfinite(xo.x) && isfinite(xo.y));
+            out[t] = xo;
+          }
+          y = yn;
+#pragma unroll
+          for (int i = 0; i < NA; ++i) u[i] = un[i];
+          info.next(k);
+        }
+      }
+#pragma unroll
+      for (int i = KV; i >= 1; --i) r[U - 1 + i] = r[i - 1];
+    }
+    cp_async_wait<0>();
+    if (bad) atomicOr(a.flags, 1u);
   }
 }
 
-// The same solve for any band within (KL, KV) = (15, 31), kl and ku read at run time.
+template <int KL, int KV, int UPW>
+__global__ void __launch_bounds__(32) k_subst_block(const __grid_constant__ SolveArgs a) {
+  extern __shared__ __align__(16) unsigned char sbuf[];
+  subst_group<KL, KV, UPW>(a, blockIdx.x, sbuf);
+}
+
+// The substitutions of many systems (the members of an ensemble) in one launch:
+// CTA b takes group b of the members' concatenated groups (member m owns groups
+// [prefix[m], prefix[m+1])); each group runs exactly the arithmetic of k_subst_block.
 template <int KL, int KV>
-__global__ void __launch_bounds__(kTpbThreads) k_subst_tpb_rt(SolveArgs a) {
-  constexpr int W1 = (KL + 2 <= 16) ? 16 : 32;  // power of 2 >= KL + 2
-  constexpr int W2 = KV + 1;
-  constexpr int S = kTpbThreads;                // slot stride
-  extern __shared__ double2 swin[];
-  const int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= a.nblk) return;  // no warp-collective operations below
-  const int T = a.Tc, kl = a.kl, kv = a.kl + a.ku, ldab = a.ldab;
-  const int cls = b % a.ncls;
-  const size_t gb = (size_t)(b >> 5) * T;
-  const double* F = a.abr + gb * ldab * 32 + (b & 31);
-  const unsigned char* P = a.dpiv + gb * 32 + (b & 31);
-  double2* X = a.work2 + gb * 32 + (b & 31);
-  const unsigned char* cflip = a.colflip_cls + (size_t)cls * T;
-  const int* ccol = a.cls_col + (size_t)cls * T;
-  double2* out = a.out + (size_t)a.act_list[b / a.ncls] * a.T;  // this system's stage output
-  bool bad = false;
-  double2* win = swin + threadIdx.x;
-  // ---- forward: positions j..j+kl in slots p mod W1 ----
-  for (int p = 0; p <= kl && p < T; ++p) win[(p & (W1 - 1)) * S] = X[(size_t)p * 32];
-  for (int j = 0; j < T - 1; ++j) {
-    const int km = min(kl, T - 1 - j);
-    double lv[KL];
-#pragma unroll
-    for (int i = 0; i < KL; ++i) lv[i] = (i < km) ? F[((size_t)j * ldab + kv + 1 + i) * 32] : 0.0;
-    const int jp = P[(size_t)j * 32];
-    const double2 inc = (j + kl + 1 < T) ? X[(size_t)(j + kl + 1) * 32] : zero2();
-    const double2 bj = win[((j + jp) & (W1 - 1)) * S];
-    if (jp) win[((j + jp) & (W1 - 1)) * S] = win[(j & (W1 - 1)) * S];
-#pragma unroll
-    for (int i = 0; i < KL; ++i) {
-      if (i < km) {
-        double2 w = win[((j + 1 + i) & (W1 - 1)) * S];
-        w.x -= lv[i] * bj.x;
-        w.y -= lv[i] * bj.y;
-        win[((j + 1 + i) & (W1 - 1)) * S] = w;
-      }
-    }
-    X[(size_t)j * 32] = bj;
-    if (j + kl + 1 < T) win[((j + kl + 1) & (W1 - 1)) * S] = inc;
+__global__ void __launch_bounds__(32) k_subst_block_multi(const SolveArgs* args, const int* prefix, int nmem) {
+  extern __shared__ __align__(16) unsigned char sbuf[];
+  const int b = blockIdx.x;
+  int lo = 0, hi = nmem - 1;  // member m with prefix[m] <= b < prefix[m+1]
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) >> 1;
+    if (prefix[mid] <= b) lo = mid;
+    else hi = mid - 1;
   }
-  if (T > 0) X[(size_t)(T - 1) * 32] = win[((T - 1) & (W1 - 1)) * S];
-  // ---- backward: x_{j+1}..x_{j+kv} in slots p mod W2 ----
-  int sj = (T - 1) % W2;  // slot of position j
-  for (int j = T - 1; j >= 0; --j) {
-    const int im = min(kv, T - 1 - j);
-    double u[KV];
-#pragma unroll
-    for (int i = 0; i < KV; ++i) u[i] = (i < im) ? F[((size_t)(j + 1 + i) * ldab + kv - 1 - i) * 32] : 0.0;
-    const double dinv = F[((size_t)j * ldab + kv) * 32];  // U's diagonal is stored as its reciprocal
-    double2 acc = X[(size_t)j * 32];
-#pragma unroll
-    for (int i = KV - 1; i >= 0; --i) {
-      if (i < im) {
-        int sl = sj + 1 + i;
-        if (sl >= W2) sl -= W2;
-        const double2 xv = win[sl * S];
-        acc.x -= u[i] * xv.x;
-        acc.y -= u[i] * xv.y;
-      }
-    }
-    const double2 xj = make_double2(acc.x * dinv, acc.y * dinv);
-    win[sj * S] = xj;
-    {  // the solution, scaled back, straight into the stage output (original order)
-      const int t = ccol[j];
-      if (t >= 0) {
-        const double2 xo = flip_col(xj, cflip[j]);
-        bad |= !(isfinite(xo.x) && isfinite(xo.y));
-        out[t] = xo;
-      }
-    }
-    sj = (sj == 0) ? W2 - 1 : sj - 1;
-  }
-  if (bad) atomicOr(a.flags, 1u);
+  const SolveArgs& a = args[lo];
+  if (a.upw == 16) subst_group<KL, KV, 16>(a, b - prefix[lo], sbuf);
+  else subst_group<KL, KV, 32>(a, b - prefix[lo], sbuf);
 }
 
 // ------------------------------------------------------------------------------
@@ -2119,6 +2292,13 @@ __global__ void __launch_bounds__(kTpbThreads) k_subst_tpb_rt(SolveArgs a) {
 // stage), K_std_i = 0.
 // ------------------------------------------------------------------------------
 constexpr int kRhsThreads = 256;
+
+// entry pc of class c of the system with slot word sl into the block layout
+__device__ __forceinline__ void store_block_rhs(const SolveArgs& a, int sl, int c, int pc, unsigned char neg, double2 v) {
+  if ((sl & kMirrorBit) && neg) v = make_double2(-v.x, -v.y);
+  sl &= kMirrorBit - 1;
+  a.work2[((size_t)(c * a.ngrp + (sl >> 5)) * a.Tc + pc) * 32 + (sl & 31)] = v;
+}
 
 __global__ void __launch_bounds__(kRhsThreads) k_rhs_nl(SolveArgs a, NLArgs n) {
   extern __shared__ double2 shr[];
@@ -2202,9 +2382,9 @@ __global__ void __launch_bounds__(kRhsThreads) k_rhs_nl(SolveArgs a, NLArgs n) {
     r = cadd(r, cscale(kh, a.ch[a.nprev]));
     if (act) {
       if (a.rowflip) r = flip_row(r, a.rowflip[t]);
-      if (a.work2) {  // thread-per-block layout, class order
-        const int pos = a.row_pos[t], c = pos >= a.Tc ? 1 : 0, bb = aidx * a.ncls + c;
-        a.work2[((size_t)(bb >> 5) * a.Tc + pos - c * a.Tc) * 32 + (bb & 31)] = r;
+      if (a.work2) {  // block layout, class order
+        const int pos = a.row_pos[t], c = pos >= a.Tc ? 1 : 0;
+        store_block_rhs(a, a.slot[sid], c, pos - c * a.Tc, a.row_neg[t], r);
       } else {
         a.work[(size_t)sid * a.wst + (a.row_pos ? a.row_pos[t] : t)] = r;
       }
@@ -2230,7 +2410,7 @@ __global__ void __launch_bounds__(kRhsThreads) k_kstd_out(SolveArgs a) {
   const int sid = a.act_list[aidx];
   const int T = a.T;
   const int kx = sid / a.d.NYA, ky = sid - kx * a.d.NYA;
-  // thread-per-block solve: the solution is already in out, original order, and
+  // block solve: the solution is already in out, original order, and
   // only K_std remains (L with its original columns); whole-system solve: the
   // solution is in work (class order = original order), copied to out here
   const bool in_out = a.work2 != nullptr;
@@ -2486,9 +2666,9 @@ __global__ void __launch_bounds__(kTileRows, 6) k_rhs_tiles(SolveArgs a, NLArgs 
   // M with the single monomial 1 (every recipe here): its coefficient is exactly
   // 1 and the complex multiply is skipped (identical for finite values)
   const bool m_unit = a.Mw.ngroups == 1 && a.Mw.gkx[0] == 0 && a.Mw.gky[0] == 0;
-  int ai[kRhsSys];
+  int ai[kRhsSys];  // slot words, -1: inactive
 #pragma unroll
-  for (int u = 0; u < kRhsSys; ++u) ai[u] = u < ns ? a.act_index[s0 + u] : -1;
+  for (int u = 0; u < kRhsSys; ++u) ai[u] = u < ns ? a.slot[s0 + u] : -1;
   cp_async_wait<0>();
   __syncthreads();
   if (!row_ok) return;  // no barrier below
@@ -2551,7 +2731,7 @@ __global__ void __launch_bounds__(kTileRows, 6) k_rhs_tiles(SolveArgs a, NLArgs 
   }
   // phase 3: stores
   const int pos = a.row_pos[t], c = pos >= a.Tc ? 1 : 0, pc = pos - c * a.Tc;
-  const unsigned char rf = a.rowflip ? a.rowflip[t] : 0;
+  const unsigned char rf = a.rowflip ? a.rowflip[t] : 0, rn = a.row_neg[t];
   bool bad = false;
 #pragma unroll
   for (int u = 0; u < kRhsSys; ++u) {
@@ -2562,8 +2742,7 @@ __global__ void __launch_bounds__(kTileRows, 6) k_rhs_tiles(SolveArgs a, NLArgs 
     double2 v = cadd(r[u], cscale(kh[u], a.ch[a.nprev]));
     if (ai[u] >= 0) {
       if (a.rowflip) v = flip_row(v, rf);
-      const int bb = ai[u] * a.ncls + c;
-      a.work2[((size_t)(bb >> 5) * a.Tc + pc) * 32 + (bb & 31)] = v;
+      store_block_rhs(a, ai[u], c, pc, rn, v);
     } else {
       if (a.last_stage) v = zero2();
       bad |= !(isfinite(v.x) && isfinite(v.y));
@@ -3365,22 +3544,24 @@ void launch_rhs_nl(const SolveArgs& a, const NLArgs& n, cudaStream_t s) {
   set_smem(k_rhs_nl, sm);
   k_rhs_nl<<<nsys, rows_threads(a.T), sm, s>>>(a, n);
 }
+template <int KL, int KV, int UPW>
+static void launch_subst_block(const SolveArgs& a, cudaStream_t s) {
+  const size_t sm = SubstShape<KL, KV, UPW>::kBytes;
+  set_smem(k_subst_block<KL, KV, UPW>, sm);
+  k_subst_block<KL, KV, UPW><<<a.ncls * a.ngrp, 32, sm, s>>>(a);
+}
 void launch_subst(const SolveArgs& a, cudaStream_t s) {
   if (a.nact <= 0) return;
   if (a.work2) {
-    if (a.nblk > 0) {
-      const int kv = a.kl + a.ku, grid = (a.nblk + kTpbThreads - 1) / kTpbThreads;
-      // band (kl, kl+ku) = (9, 23) of the plane-layer recipes compiled, any other
-      // band within (15, 31) through the run-time-band kernel
-      if (!a.subst_rt && a.kl == 9 && kv == 23 && a.ldab == 34) {
-        const size_t sm = (size_t)kTpbThreads * 24 * sizeof(double2);
-        set_smem(k_subst_tpb<9, 23, 34>, sm);
-        k_subst_tpb<9, 23, 34><<<grid, kTpbThreads, sm, s>>>(a);
-      } else {
-        const size_t sm = (size_t)kTpbThreads * 32 * sizeof(double2);
-        set_smem(k_subst_tpb_rt<15, 31>, sm);
-        k_subst_tpb_rt<15, 31><<<grid, kTpbThreads, sm, s>>>(a);
-      }
+    // the band (kl, kl+ku) = (9, 23) of the plane-layer recipes compiled, any
+    // other band within (15, 31) through the wider instance
+    const bool plane = !a.subst_rt && a.kl == 9 && a.kl + a.ku == 23;
+    if (a.upw == 16) {
+      if (plane) launch_subst_block<9, 23, 16>(a, s);
+      else launch_subst_block<15, 31, 16>(a, s);
+    } else {
+      if (plane) launch_subst_block<9, 23, 32>(a, s);
+      else launch_subst_block<15, 31, 32>(a, s);
     }
     return;
   }
@@ -3390,18 +3571,13 @@ void launch_subst(const SolveArgs& a, cudaStream_t s) {
   k_subst_real<32><<<(a.nact + kWPBr - 1) / kWPBr, kWPBr * 32, sm, s>>>(a);
 }
 bool subst_multi_supported(const SolveArgs& a) {
-  return a.work2 && a.nblk > 0 && a.kl == 9 && a.kl + a.ku == 23 && a.ldab == 34;
+  return a.work2 && a.ngrp > 0 && a.kl == 9 && a.kl + a.ku == 23;
 }
-void launch_subst_multi(const SolveArgs* d_args, const long long* d_prefix, int nmem, long long total,
-                        cudaStream_t s) {
+void launch_subst_multi(const SolveArgs* d_args, const int* d_prefix, int nmem, int total, bool wide, cudaStream_t s) {
   if (total <= 0) return;
-  const size_t sm = (size_t)kTpbThreads * 24 * sizeof(double2);
-  set_smem(k_subst_tpb_multi<9, 23, 34>, sm);
-  static int nct = 0;
-  if (!nct) nct = persistent_ctas(k_subst_tpb_multi<9, 23, 34>, kTpbThreads, sm);
-  const long long need = (total + kTpbThreads - 1) / kTpbThreads;
-  k_subst_tpb_multi<9, 23, 34><<<(int)std::min<long long>(nct, need), kTpbThreads, sm, s>>>(d_args, d_prefix, nmem,
-                                                                                          total);
+  const size_t sm = wide ? SubstShape<9, 23, 32>::kBytes : SubstShape<9, 23, 16>::kBytes;
+  set_smem(k_subst_block_multi<9, 23>, sm);
+  k_subst_block_multi<9, 23><<<total, 32, sm, s>>>(d_args, d_prefix, nmem);
 }
 void launch_kstd_out(const SolveArgs& a, cudaStream_t s) {
   if (a.nact <= 0) return;
@@ -3434,7 +3610,7 @@ void launch_solve_real(const SolveArgs& a, const NLArgs& n, cudaStream_t s) {
 void launch_factor_real(const FactorArgs& a, cudaStream_t s) {
   if (a.nact <= 0) return;
   if (a.tpb) {
-    const int nb = a.ncls * a.nact;
+    const int nb = a.ncls * a.ngrp * a.upw;
     // the shared-memory window kernel when a warp's (or at least one thread's)
     // windows fit in a CTA's shared memory, else the in-place kernel
     int dev = 0, smax = 0;
@@ -3452,11 +3628,11 @@ void launch_factor_real(const FactorArgs& a, cudaStream_t s) {
     } else {
       k_factor_tpb<<<(nb + kTpbThreads - 1) / kTpbThreads, kTpbThreads, 0, s>>>(a);
     }
-    if (a.cmask && a.ldab <= 64 && a.kl + a.ku <= 32 && a.kl <= 32) {
-      cudaMemsetAsync(a.cmask, 0, (size_t)a.Tc * sizeof(unsigned long long), s);
-      k_mask_cols<<<dim3((nb + 31) / 32, (a.Tc + 7) / 8), 256, 0, s>>>(a);
-      k_mask_rows<<<(a.Tc + 127) / 128, 128, 0, s>>>(a);
-    }
+    const int ng = a.ncls * a.ngrp;
+    cudaMemsetAsync(a.cmask, 0, (size_t)a.ncls * a.Tc * sizeof(unsigned long long), s);
+    k_mask_cols<<<dim3(ng, (a.Tc + 7) / 8), 256, 0, s>>>(a);
+    k_pack_info<<<a.ncls, 32, 0, s>>>(a);
+    k_pack<<<dim3(ng, (a.Tc + 7) / 8), 256, 0, s>>>(a);
     return;
   }
   k_factor_real<<<dim3((a.nact + kWPB - 1) / kWPB, a.ncls), kWPB * 32, 0, s>>>(a);

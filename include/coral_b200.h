@@ -75,6 +75,8 @@ typedef struct coral_handle coral_handle;
                                         (L and U entries nonzero in some block, and the diagonal),
                                         summed over the block's columns; 0 before coral_factorize or
                                         when the solve reads the whole band */
+#define CORAL_Q_SYS_FACTOR_UNITS 1300   /* + isys: LU factorisations held: one per active system, or one per
+                                        (kx, ky), (kx, -ky) pair where the recipe has that symmetry */
 
 /*
  * Create a solver from the text of coral.equations and coral.parameters.in.
@@ -351,7 +353,7 @@ int coral_set_penalisation_mask(coral_handle* h, const double* mask);
  * scheme's stage count may not) advanced together on one CUDA stream with one
  * CUDA graph per step.  Per stage the band substitutions of every member's
  * (kx, ky) systems run as one persistent launch when every member's systems
- * use the split thread-per-block layout with the plane-layer band (9, 23)
+ * use the split block layout with the plane-layer band (9, 23)
  * (coral_ensemble_query(e, 2) = 1); otherwise member by member.  The
  * reference runs one problem per job and solves its systems one at a time
  * (src/plane_layer/PL_algebra_z_3D.f90:197-214); each member here computes

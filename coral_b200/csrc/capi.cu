@@ -289,6 +289,10 @@ struct coral_handle {
   std::string err;
   int device = 0;
   cudaStream_t stream = nullptr;
+  // the mean systems of a stage run beside the (kx, ky) solves, on a stream forked
+  // after the forward transforms and joined at the stage's end
+  cudaStream_t zstream = nullptr;
+  cudaEvent_t zfork = nullptr, zjoin = nullptr;
   cudaStream_t ystream[kYStreams] = {};
   cudaEvent_t yfork = nullptr, yjoin[kYStreams] = {};
   Parameters P;
@@ -621,6 +625,9 @@ void setup(coral_handle* h, const std::string& eqs, const std::string& pars, con
   h->device = device;
   CK(cudaSetDevice(device));
   CK(cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking));
+  CK(cudaStreamCreateWithFlags(&h->zstream, cudaStreamNonBlocking));
+  CK(cudaEventCreateWithFlags(&h->zfork, cudaEventDisableTiming));
+  CK(cudaEventCreateWithFlags(&h->zjoin, cudaEventDisableTiming));
   h->P = parse_parameters(pars);
   h->R = parse_equations(eqs, h->smagorinsky);
   h->TB = ars_tableau(scheme && *scheme ? std::string(scheme) : h->P.scheme);
@@ -1234,6 +1241,25 @@ SolveArgs make_solve_args(coral_handle* h, KSys& k, int i, double dt) {
   return sa;
 }
 
+// Stage i of the mean systems (marching.f90:83-107, 372-397) on stream s: from the
+// stage's qspec, independent of the (kx, ky) systems.
+int launch_mean_systems(coral_handle* h, int i, double dt, cudaStream_t s) {
+  if (h->zs.empty()) return 0;
+  ZeroArgs za{};
+  za.nsys = (int)h->zs.size();
+  for (size_t k = 0; k < h->zs.size(); ++k) za.sys[k] = h->zs[k].dev;
+  za.qspec = h->qspec;
+  za.d = h->d;
+  za.stage = i;
+  for (int j = 0; j <= i; ++j) {
+    za.ca[j] = (j < i) ? dt * h->TB.a(i, j) : 0.0;
+    za.ch[j] = dt * h->TB.ahat(i + 1, j);
+  }
+  za.last_stage = (i == h->TB.stages - 1) ? 1 : 0;
+  launch_zero_step(za, s);
+  return 1;
+}
+
 // Stage i of one_step_beyond (marching.f90:9-28) in three phases, so that an
 // ensemble can run the band substitutions of all its members as one launch:
 //   pre   full variables -> physical space, products, forward transforms
@@ -1360,6 +1386,16 @@ int enqueue_stage_pre(coral_handle* h, int i, double dt, PhaseTimer* pt) {
     launch_remove_zmean(d, h->qspec + (size_t)q * d.NXH * d.NYA * d.NZ, h->stream);
     ++nl;
   }
+  // The mean systems' step (one warp per system, 40-140 us of serial sweeps) needs
+  // only qspec: beside the solves it costs nothing (in line with them 0.08 of 0.53
+  // ms per step at 64^2 x 48, 0.28 of 4.6 at 128^2 x 192).  Eager phase timing keeps
+  // it in line.
+  if (!pt && !h->zs.empty()) {
+    CK(cudaEventRecord(h->zfork, h->stream));
+    CK(cudaStreamWaitEvent(h->zstream, h->zfork, 0));
+    nl += launch_mean_systems(h, i, dt, h->zstream);
+    CK(cudaEventRecord(h->zjoin, h->zstream));
+  }
   for (auto& k : h->ks) {
     NLArgs na = make_nl_args(h, k, i);
     SolveArgs sa = make_solve_args(h, k, i, dt);
@@ -1390,8 +1426,6 @@ int enqueue_stage_subst(coral_handle* h, int i, double dt, PhaseTimer* pt) {
 
 int enqueue_stage_post(coral_handle* h, int i, double dt, PhaseTimer* pt) {
   int nl = 0;
-  const int S = h->TB.stages;
-  const bool last = (i == S - 1);
   for (auto& k : h->ks)
     if (k.real) {
       SolveArgs sa = make_solve_args(h, k, i, dt);
@@ -1401,21 +1435,13 @@ int enqueue_stage_post(coral_handle* h, int i, double dt, PhaseTimer* pt) {
       ++nl;
     }
   if (!h->zs.empty()) {
-    ZeroArgs za{};
-    za.nsys = (int)h->zs.size();
-    for (size_t s = 0; s < h->zs.size(); ++s) za.sys[s] = h->zs[s].dev;
-    za.qspec = h->qspec;
-    za.d = h->d;
-    za.stage = i;
-    for (int j = 0; j <= i; ++j) {
-      za.ca[j] = (j < i) ? dt * h->TB.a(i, j) : 0.0;
-      za.ch[j] = dt * h->TB.ahat(i + 1, j);
+    if (pt) {
+      pt->begin(8);
+      nl += launch_mean_systems(h, i, dt, h->stream);
+      pt->end();
+    } else {
+      CK(cudaStreamWaitEvent(h->stream, h->zjoin, 0));
     }
-    za.last_stage = last ? 1 : 0;
-    if (pt) pt->begin(8);
-    launch_zero_step(za, h->stream);
-    if (pt) pt->end();
-    ++nl;
   }
   return nl;
 }
@@ -2113,6 +2139,11 @@ void release_streams(coral_handle* h) {
   }
   if (h->yfork) cudaEventDestroy(h->yfork);
   h->yfork = nullptr;
+  if (h->zstream) cudaStreamDestroy(h->zstream);
+  if (h->zfork) cudaEventDestroy(h->zfork);
+  if (h->zjoin) cudaEventDestroy(h->zjoin);
+  h->zstream = nullptr;
+  h->zfork = h->zjoin = nullptr;
   if (h->stream) cudaStreamDestroy(h->stream);
   h->stream = nullptr;
 }

@@ -424,6 +424,11 @@ FftPlan make_plan(DevAlloc& mem, int N) {
     tw[k] = make_double2((double)cosl(a), (double)sinl(a));
   }
   p.tw = mem.upload(tw);
+  for (int pv = 0; pv < 2; ++pv) {
+    std::vector<double2> t(pass_tw_len(N, pv));
+    for (size_t i = 0; i < t.size(); ++i) t[i] = tw[pass_tw_index(N, pv, (int)i)];
+    p.tws[pv] = mem.upload(t);
+  }
   return p;
 }
 

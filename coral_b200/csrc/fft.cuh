@@ -14,7 +14,8 @@ struct FftPlan {
   int N;
   int nst;
   int radix[16];
-  const double2* tw;  // tw[k] = exp(-2 pi i k / N), k < N
+  const double2* tw;      // tw[k] = exp(-2 pi i k / N), k < N (plans chosen at run time)
+  const double2* tws[2];  // the compiled plans' twiddles pass by pass (pass_tw_index), per plan variant
 };
 
 __device__ __forceinline__ double2 cadd(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
@@ -315,33 +316,66 @@ __device__ __forceinline__ void dft(double2 (&x)[R]) {
   }
 }
 
-// Twiddles of the second pass of a two-pass plan N = R0 x R1, laid out [k][r - 1]
-// (k < R0, 1 <= r < R1): t[k (R1 - 1) + r - 1] = exp(-2 pi i r k / N).  For a
-// fixed r, consecutive k are R1 - 1 16-byte words apart, an odd number for the
-// even R1 of the two-pass plans, so the 16-byte reads of 8 consecutive k fall in
-// 8 distinct bank groups (the N-entry table read at r k conflicts up to 8-way).
-template <int N, int PV>
-__host__ __device__ constexpr int tw_pass2_len() {
-  return plan_of(N, PV).nst == 2 ? plan_of(N, PV).r[0] * (plan_of(N, PV).r[1] - 1) : 0;
+// Twiddles of the passes S >= 1 of a compiled plan, one table [r - 1][k] after the
+// other: entry (r, k), 1 <= r < R, k < Ns (the product of the earlier radices), is
+// exp(-2 pi i r k / (Ns R)).  Consecutive lanes take consecutive k, so a load touches
+// consecutive 16-byte words (the N-entry table read at stride r touched up to a
+// line per lane).  With the padding below, per step at 384^2 x 192: inverse y
+// 2.91 -> 2.48 ms, inverse x 2.38 -> 2.20, forward x 3.48 -> 3.16, forward y 3.59
+// -> 3.38, z 9.3 -> 9.07; z at 96 points 0.54 -> 0.46 ms.
+__host__ __device__ constexpr int pass_ns(int N, int PV, int S) {
+  int ns = 1;
+  for (int q = 0; q < S; ++q) ns *= plan_of(N, PV).r[q];
+  return ns;
 }
-template <int N, int PV>
-__device__ __forceinline__ void build_tw_pass2(double2* t, const double2* tw) {
-  constexpr PlanR P = plan_of(N, PV);
-  static_assert(P.nst == 2 && (P.r[1] % 2) == 0, "two-pass plan with an even second radix");
-  constexpr int R0 = P.r[0], R1 = P.r[1];
-  for (int i = threadIdx.x; i < R0 * (R1 - 1); i += blockDim.x) {
-    const int k = i / (R1 - 1), r = i - k * (R1 - 1) + 1;
-    t[i] = tw[r * k];  // N = R0 R1: the pass's twiddle stride is 1
+__host__ __device__ constexpr int pass_tw_offset(int N, int PV, int S) {
+  int o = 0;
+  for (int q = 1; q < S; ++q) o += pass_ns(N, PV, q) * (plan_of(N, PV).r[q] - 1);
+  return o;
+}
+__host__ __device__ constexpr int pass_tw_len(int N, int PV) { return pass_tw_offset(N, PV, plan_of(N, PV).nst); }
+// index into the N-entry table of entry i of the pass tables
+__host__ __device__ inline int pass_tw_index(int N, int PV, int i) {
+  const PlanR p = plan_of(N, PV);
+  int ns = 1;
+  for (int s = 0; s < p.nst; ++s) {
+    const int n = s == 0 ? 0 : ns * (p.r[s] - 1);
+    if (i < n) return (i / ns + 1) * (i % ns) * (N / (ns * p.r[s]));
+    i -= n;
+    ns *= p.r[s];
   }
+  return 0;
+}
+
+// Padding of a line between the first and the second pass of a two-pass plan whose
+// first radix is even: its butterflies store R0 consecutive elements each, so 8
+// lanes' 16-byte stores at stride R0 would share banks; one element is left out
+// after every pad_every butterflies (LINE_FAST: 4 interleaved lines x 2
+// butterflies).  Odd radices need none, and later passes store in natural order.
+__host__ __device__ constexpr int pad_every(int N, int PV, bool line_fast) {
+  const PlanR p = plan_of(N, PV);
+  if (p.nst != 2 || p.r[0] % 2) return 0;
+  if (line_fast) return 1;
+  return p.r[0] % 8 == 0 ? 1 : p.r[0] % 4 == 0 ? 2 : 4;
+}
+__host__ __device__ constexpr int line_len(int N, int PV, bool line_fast) {
+  const int e = N ? pad_every(N, PV, line_fast) : 0;
+  return e ? N + (N / plan_of(N, PV).r[0] - 1) / e : N;
+}
+// line stride of the passes that walk 4 interleaved lines: 2 mod 8, so that the
+// same position of the lines hits 4 distinct even 16-byte bank groups
+__host__ __device__ constexpr int line_stride(int N, int PV) {
+  const int n = line_len(N, PV, true);
+  return n == N ? N + 2 : (n + 5) / 8 * 8 + 2;
 }
 
 // One in-place pass of radix R over nl lines (line stride LS) by NT threads;
-// NLMAX bounds nl (registers hold ceil(NLMAX N / (R NT)) butterflies per thread).
-// TWL: tw is the [k][r - 1] table of build_tw_pass2 (second pass of a two-pass plan).
-template <int N, int R, int Ns, bool INV, int NT, int NLMAX, bool TWL = false>
+// NLMAX bounds nl (registers hold ceil(NLMAX N / (R NT)) butterflies per thread);
+// tw: the pass's table; PADE: pad_every of the line as the first pass left it.
+template <int N, int R, int Ns, bool INV, int NT, int NLMAX, int PADE = 0>
 __device__ __forceinline__ void fft_pass(double2* A, int nl, int LS, const double2* __restrict__ tw) {
   constexpr int NB = N / R;               // butterflies per line
-  constexpr int TS = N / (Ns * R);        // twiddle stride
+  static_assert(PADE == 0 || NB == Ns, "padding: second of two passes");
   constexpr int BPT = (NLMAX * NB + NT - 1) / NT;
   const int total = nl * NB;
   double2 v[BPT][R];
@@ -352,12 +386,12 @@ __device__ __forceinline__ void fft_pass(double2* A, int nl, int LS, const doubl
       const int line = b / NB, j = b - line * NB;
       const double2* sl = A + line * LS + j;
 #pragma unroll
-      for (int r = 0; r < R; ++r) v[i][r] = sl[r * NB];
+      for (int r = 0; r < R; ++r) v[i][r] = sl[r * NB + (PADE ? r / PADE : 0)];
       if constexpr (Ns > 1) {
         const int k = j % Ns;
 #pragma unroll
         for (int r = 1; r < R; ++r) {
-          double2 w = TWL ? tw[k * (R - 1) + r - 1] : tw[r * k * TS];
+          double2 w = tw[(r - 1) * Ns + k];
           if (INV) w = cconj(w);
           v[i][r] = cmul(v[i][r], w);
         }
@@ -386,9 +420,9 @@ __device__ __forceinline__ void fft_pass(double2* A, int nl, int LS, const doubl
 // LINE_FAST: consecutive threads take consecutive lines at the same position
 // (so that interleaved lines of a global array load together); otherwise
 // consecutive positions of one line.
-template <int N, int R, bool INV, int NT, int NLMAX, bool LINE_FAST, class Load>
+template <int N, int R, bool INV, int NT, int NLMAX, bool LINE_FAST, int PV, class Load>
 __device__ __forceinline__ void fft_pass_first(double2* A, int nl, int LS, Load&& ld) {
-  constexpr int NB = N / R;
+  constexpr int NB = N / R, PADE = pad_every(N, PV, LINE_FAST);
   constexpr int BPT = (NLMAX * NB + NT - 1) / NT;
   const int total = nl * NB;
 #pragma unroll
@@ -401,7 +435,7 @@ __device__ __forceinline__ void fft_pass_first(double2* A, int nl, int LS, Load&
 #pragma unroll
       for (int r = 0; r < R; ++r) v[r] = ld(line, j + r * NB);
       dft<R, INV>(v);
-      double2* dl = A + line * LS + j * R;
+      double2* dl = A + line * LS + j * R + (PADE ? j / PADE : 0);
 #pragma unroll
       for (int r = 0; r < R; ++r) dl[r] = v[r];
     }
@@ -409,25 +443,25 @@ __device__ __forceinline__ void fft_pass_first(double2* A, int nl, int LS, Load&
   __syncthreads();
 }
 
-template <int N, int S, int Ns, bool INV, int NT, int NLMAX, int PV = 0, bool TWL = false>
+// passes S, S + 1, ... of plan variant PV; tw: the plan's pass tables; PADE as
+// fft_pass's (of pass 1)
+template <int N, int S, int Ns, bool INV, int NT, int NLMAX, int PV = 0, int PADE = 0>
 __device__ __forceinline__ void fft_passes(double2* A, int nl, int LS, const double2* tw) {
   constexpr PlanR P = plan_of(N, PV);
-  static_assert(!TWL || P.nst == 2, "the pass-2 twiddle table belongs to two-pass plans");
   if constexpr (S < P.nst) {
     constexpr int R = P.r[S];
-    fft_pass<N, R, Ns, INV, NT, NLMAX, TWL>(A, nl, LS, tw);
-    fft_passes<N, S + 1, Ns * R, INV, NT, NLMAX, PV, TWL>(A, nl, LS, tw);
+    fft_pass<N, R, Ns, INV, NT, NLMAX, S == 1 ? PADE : 0>(A, nl, LS, tw + pass_tw_offset(N, PV, S));
+    fft_passes<N, S + 1, Ns * R, INV, NT, NLMAX, PV, PADE>(A, nl, LS, tw);
   }
 }
 
-// Batched FFT of nl <= NLMAX lines (line stride LS) by NT threads: compile-time
-// length NC in place in A (B unused), or the runtime plan (NC == 0) ping-ponging
-// through B.  Returns the buffer holding the result.  The caller synchronises
-// before (inputs written) and may read the result directly after.
-// The same with the inputs produced by ld(line, k) (see fft_pass_first); the
-// caller need not synchronise before.  Runtime plans stage the inputs in A first.
-// TWL: p.tw is the table of build_tw_pass2 (compiled two-pass plans only).
-template <int NC, bool INV, int NT, int NLMAX, bool LINE_FAST = false, int PV = 0, bool TWL = false, class Load>
+// Batched FFT of nl <= NLMAX lines (line stride LS >= line_len) by NT threads:
+// compile-time length NC in place in A (B unused), or the runtime plan (NC == 0)
+// ping-ponging through B.  Returns the buffer holding the result.  The inputs are
+// produced by ld(line, k) (see fft_pass_first; runtime plans stage them in A
+// first), so the caller need not synchronise before; it may read the result
+// directly after.
+template <int NC, bool INV, int NT, int NLMAX, bool LINE_FAST = false, int PV = 0, class Load>
 __device__ __forceinline__ double2* fft_lines_ld(double2* A, double2* B, int nl, int LS, const FftPlan& p,
                                                  Load&& ld) {
   if constexpr (NC == 0) {
@@ -440,19 +474,20 @@ __device__ __forceinline__ double2* fft_lines_ld(double2* A, double2* B, int nl,
   } else {
     constexpr PlanR P = plan_of(NC, PV);
     static_assert(P.nst > 0, "transform length must be 2^a 3^b");
-    fft_pass_first<NC, P.r[0], INV, NT, NLMAX, LINE_FAST>(A, nl, LS, ld);
-    fft_passes<NC, 1, P.r[0], INV, NT, NLMAX, PV, TWL>(A, nl, LS, p.tw);
+    fft_pass_first<NC, P.r[0], INV, NT, NLMAX, LINE_FAST, PV>(A, nl, LS, ld);
+    fft_passes<NC, 1, P.r[0], INV, NT, NLMAX, PV, pad_every(NC, PV, LINE_FAST)>(A, nl, LS, p.tws[PV]);
     return A;
   }
 }
 
+// The same of lines already in A (unpadded; the caller has synchronised)
 template <int NC, bool INV, int NT, int NLMAX>
 __device__ __forceinline__ double2* fft_lines_n(double2* A, double2* B, int nl, int LS, const FftPlan& p) {
   if constexpr (NC == 0) {
     return fft_lines<INV>(A, B, nl, LS, p);
   } else {
     static_assert(make_planr(NC).nst > 0, "transform length must be 2^a 3^b");
-    fft_passes<NC, 0, 1, INV, NT, NLMAX>(A, nl, LS, p.tw);
+    fft_passes<NC, 0, 1, INV, NT, NLMAX>(A, nl, LS, p.tws[0]);
     return A;
   }
 }

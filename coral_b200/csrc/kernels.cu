@@ -29,10 +29,7 @@ constexpr int kNB2 = 8;  // n lines per CTA, x passes (packed in pairs)
 constexpr int kXB3 = 16; // x columns per CTA, inverse z pass (packed in pairs)
 constexpr int kQC = 5;   // quadratic variables per FFT batch, forward z pass (one radix-9 / radix-8
                          // butterfly per thread at NZAA = 288)
-constexpr int kPadY = 2;   // line stride of the y passes (kNB1 interleaved lines)
-constexpr int kPadXY = 2;  // line stride N + 2 in the x / y passes, whose loads and stores
-                           // walk 4 interleaved lines: 2 line + position hits 8 distinct
-                           // 16-byte bank groups
+constexpr int kPadRt = 2;  // line stride N + 2 of the x / y passes with run-time plans
 constexpr int kThreads = 256;
 // FFT plans of the time-step transforms (fft.cuh plan_of): the x passes and the
 // fused z passes use the two-pass plans (576 = 24 x 24, 288 = 18 x 16); the y
@@ -113,7 +110,7 @@ __global__ void __launch_bounds__(kThreadsY, kMinBlocksY) k_inv_y(Dims d, const 
                                                      const double* kyv, double2* Y1, FftPlan py) {
   extern __shared__ double2 sm[];
   const int f = blockIdx.x, n0 = blockIdx.y * kNB1, kx = blockIdx.z;
-  const int NYA = NF ? NF : d.NYA, LS = NYA + kPadY;
+  const int NYA = NF ? NF : d.NYA, LS = NF ? line_stride(NF, kPlanY) : NYA + kPadRt;
   double2* A = sm;
   double2* B = sm + kNB1 * LS;  // runtime plan only
   // the CTA's build tables in shared memory: per term and line the stencil's
@@ -210,7 +207,7 @@ __global__ void __launch_bounds__(kThreadsY, kMinBlocksY) k_inv_y1(Dims d, const
                                                       const double* kxv, const double* kyv, double2* Y1, FftPlan py) {
   extern __shared__ double2 sm[];
   const int f = blockIdx.x, n0 = blockIdx.y * kNB1, kx = blockIdx.z;
-  const int NYA = NF ? NF : d.NYA, LS = NYA + kPadY;
+  const int NYA = NF ? NF : d.NYA, LS = NF ? line_stride(NF, kPlanY) : NYA + kPadRt;
   double2* A = sm;
   double2* B = sm + kNB1 * LS;  // runtime plan only
   __shared__ int s_tt[kNB1][kTabW];
@@ -294,7 +291,7 @@ __global__ void __launch_bounds__(kThreadsX, hot_min_blocks(kThreadsX)) k_inv_x(
                                                                                int y0) {
   extern __shared__ double2 sm[];
   const int f = blockIdx.x, n0 = blockIdx.y * kNB2, y = y0 + blockIdx.z;
-  const int NXA = NF ? NF : d.NXA, NP = kNB2 / 2, LS = NXA + kPadXY;
+  const int NXA = NF ? NF : d.NXA, NP = kNB2 / 2, LS = NF ? line_stride(NF, PV) : NXA + kPadRt;
   double2* A = sm;
   double2* B = sm + NP * LS;  // runtime plan only
   // position p of line m (Chebyshev pair na, na+1): the Hermitian extension of
@@ -334,8 +331,7 @@ __global__ void __launch_bounds__(kThreadsX, hot_min_blocks(kThreadsX)) k_inv_x(
 // the current tile's second FFT pass and stores run (the first pass reads the
 // staging buffer and frees it).  Staging rows are kNB2 + 1 16-byte words apart,
 // so that the first pass's reads (4 lines x 2 positions a quarter warp) fall in
-// distinct bank groups; the second pass reads its twiddles from the
-// conflict-free table of build_tw_pass2.  Shared memory (line buffer, staging,
+// distinct bank groups; the twiddles are in shared memory.  That (line buffer, staging,
 // table) admits 3 CTAs per SM at NXAA = 576: registers are sized for 3.
 constexpr int kStgX = kNB2 + 1;
 #define kThreadsXP xy_threads(NF, kNB2 / 2, 1)
@@ -344,17 +340,17 @@ __global__ void __launch_bounds__(kThreadsXP, 3) k_inv_x_pipe(Dims d, int nf, co
                                                                                       double* Y2, FftPlan px) {
   constexpr int NT = kThreadsXP, NXA = NF, NP = kNB2 / 2;
   constexpr PlanR P = plan_of(NF, 1);
-  constexpr int kTw2 = tw_pass2_len<NF, 1>();
-  static_assert(kTw2 > 0, "two-pass plan");
+  constexpr int kTw2 = pass_tw_len(NF, 1);
+  static_assert(P.nst == 2, "two-pass plan");
   extern __shared__ double2 sm[];
   __shared__ double2 s_tw[kTw2];
-  const int LS = NXA + kPadXY;
+  constexpr int LS = line_stride(NF, 1);
   double2* A = sm;               // NP lines, stride LS
   double2* stg = A + NP * LS;    // staged input [kx][kStgX]
   const int NXH = d.NXH, NZ = d.NZ;
   const int nnb = (NZ + kNB2 - 1) / kNB2;
   const int ntiles = nf * nnb * d.NYA;
-  build_tw_pass2<NF, 1>(s_tw, px.tw);  // read after the loop's first barrier
+  for (int i = threadIdx.x; i < kTw2; i += NT) s_tw[i] = px.tws[1][i];  // read after the loop's first barrier
   auto issue = [&](int tile) {
     if (tile < ntiles) {
       const int f = tile % nf, r = tile / nf, nb = r % nnb, y = r / nnb, n0 = nb * kNB2;
@@ -381,9 +377,9 @@ __global__ void __launch_bounds__(kThreadsXP, 3) k_inv_x_pipe(Dims d, int nf, co
       if (p == 0) return make_double2(a.x, b.x);
       return lo ? make_double2(a.x - b.y, a.y + b.x) : make_double2(a.x + b.y, b.x - a.y);
     };
-    fft_pass_first<NF, P.r[0], true, NT, NP, true>(A, NP, LS, ld);  // ends with a barrier
+    fft_pass_first<NF, P.r[0], true, NT, NP, true, 1>(A, NP, LS, ld);  // ends with a barrier
     issue(tile + gridDim.x);
-    fft_passes<NF, 1, P.r[0], true, NT, NP, 1, true>(A, NP, LS, s_tw);
+    fft_passes<NF, 1, P.r[0], true, NT, NP, 1, pad_every(NF, 1, true)>(A, NP, LS, s_tw);
     double* dst0 = Y2 + ((size_t)f * d.NYA + y) * NXA * NZ;
     for (int idx = threadIdx.x; idx < NP * NXA; idx += NT) {
       const int m = idx % NP, x = idx / NP, na = n0 + 2 * m;
@@ -603,6 +599,7 @@ __global__ void __launch_bounds__(kThreadsZF, z_min_blocks(NF, FB)) k_z_fused(Di
   const size_t cta = (size_t)y * gridDim.x + blockIdx.x;  // row of the KE and timeseries partial sums
   // compiled lengths: NZAA = 3 NZ / 2 (the launcher checks it)
   const int N = NF ? NF : d.NZA, NZ = NF ? 2 * NF / 3 : d.NZ;
+  const int LZ = NF ? line_len(NF, kPlanHot, false) : N;  // line stride
   const int nq = q.nq;
   const size_t vstride = (size_t)d.NYA * d.NXA * NZ;  // between variables of Y2 / Q2
   const size_t col0 = ((size_t)y * d.NXA + x0) * NZ;  // column x0 of variable 0
@@ -610,29 +607,23 @@ __global__ void __launch_bounds__(kThreadsZF, z_min_blocks(NF, FB)) k_z_fused(Di
     qv[0][threadIdx.x] = q.v1[threadIdx.x];
     qv[1][threadIdx.x] = q.v2[threadIdx.x];
   }
-  // compiled lengths: the FFT and DCT twiddles in shared memory; with a
-  // two-pass plan the FFT twiddles as the bank-conflict-free pass-2 table
-  constexpr int kTw2 = NF ? tw_pass2_len<NF, kPlanHot>() : 0;
-  constexpr bool kTwl = kTw2 > 0;
-  __shared__ double2 s_tw[kTwl ? kTw2 : (NF ? NF : 1)], s_dtw[NF ? NF : 1];
+  // compiled lengths: the FFT's pass tables and the DCT twiddles in shared memory
+  constexpr int kTw = NF ? pass_tw_len(NF, kPlanHot) : 0;
+  __shared__ double2 s_tw[kTw ? kTw : 1], s_dtw[NF ? NF : 1];
   FftPlan pzl = pz;
   const double2* dtw = dct_tw;
   if constexpr (NF != 0) {
-    if constexpr (kTwl) {
-      build_tw_pass2<NF, kPlanHot>(s_tw, pz.tw);
-    } else {
-      for (int i = threadIdx.x; i < NF; i += blockDim.x) s_tw[i] = pz.tw[i];
-    }
+    for (int i = threadIdx.x; i < kTw; i += blockDim.x) s_tw[i] = pz.tws[kPlanHot][i];
     for (int i = threadIdx.x; i < NF; i += blockDim.x) s_dtw[i] = dct_tw[i];
-    pzl.tw = s_tw;
+    pzl.tws[kPlanHot] = s_tw;
     dtw = s_dtw;
   }
   // line l of a batch: variable l / kZPairs, column pair l % kZPairs (columns
   // x0 + 2p (re) and x0 + 2p + 1 (im))
   auto col_ok = [&](int c) { return x0 + c < d.NXA; };
   double2* Fv = sm;                   // nf * kZPairs lines of the full variables
-  double2* A = Fv + nf * kZPairs * N; // FB lines of quadratic variables
-  double2* B = A + FB * N;            // runtime plan only (max(kZLines, FB) lines)
+  double2* A = Fv + nf * kZPairs * LZ; // FB lines of quadratic variables
+  double2* B = A + FB * LZ;           // runtime plan only (max(kZLines, FB) lines)
   // ---- inverse: X_n and X_{N-n} of both columns, twiddled, packed as va + i vb,
   //      produced inside the first FFT pass ----
   __syncthreads();  // qv
@@ -651,9 +642,9 @@ __global__ void __launch_bounds__(kThreadsZF, z_min_blocks(NF, FB)) k_z_fused(Di
       const double2 vb = cmul(w, make_double2(b0, -b1));
       return make_double2(va.x - vb.y, va.y + vb.x);
     };
-    const double2* R = fft_lines_ld<NF, true, NT, kZLines, false, kPlanHot, kTwl>(Fv + l0 * N, B, nl, N, pzl, ld);
-    if (R != Fv + l0 * N) {  // runtime plan with the result in the scratch lines
-      for (int idx = threadIdx.x; idx < nl * N; idx += blockDim.x) Fv[l0 * N + idx] = R[idx];
+    const double2* R = fft_lines_ld<NF, true, NT, kZLines, false, kPlanHot>(Fv + l0 * LZ, B, nl, LZ, pzl, ld);
+    if (R != Fv + l0 * LZ) {  // runtime plan with the result in the scratch lines
+      for (int idx = threadIdx.x; idx < nl * N; idx += blockDim.x) Fv[l0 * LZ + idx] = R[idx];
       __syncthreads();
     }
   }
@@ -673,7 +664,7 @@ __global__ void __launch_bounds__(kThreadsZF, z_min_blocks(NF, FB)) k_z_fused(Di
           if (col_ok(2 * pr)) a = src[at];
           if (col_ok(2 * pr + 1)) b = src[at + N];
         }
-        Fv[(f * kZPairs + pr) * N + m] = make_double2(a, b);
+        Fv[(f * kZPairs + pr) * LZ + m] = make_double2(a, b);
       }
     }
     __syncthreads();
@@ -691,7 +682,7 @@ __global__ void __launch_bounds__(kThreadsZF, z_min_blocks(NF, FB)) k_z_fused(Di
 #pragma unroll
       for (int j = 0; j < 3; ++j)
         if (j < ncf) {
-          const double2 v = Fv[(j * kZPairs + pr) * N + m];
+          const double2 v = Fv[(j * kZPairs + pr) * LZ + m];
           const double s = (j == 2) ? wzinv[z] : 1.0;
           double a = oka ? fabs(v.x) * s : 0.0;
           if (okb) a = fmax(a, fabs(v.y) * s);
@@ -706,11 +697,11 @@ __global__ void __launch_bounds__(kThreadsZF, z_min_blocks(NF, FB)) k_z_fused(Di
           const int v1 = qv[0][qg], v2 = qv[1][qg];
           double pa, pb;
           if (v1 < 0 || v2 < 0) {
-            const double2 f1 = Fv[((v1 < 0 ? v2 : v1) * kZPairs + pr) * N + m];
+            const double2 f1 = Fv[((v1 < 0 ? v2 : v1) * kZPairs + pr) * LZ + m];
             pa = f1.x;
             pb = f1.y;
           } else {
-            const double2 f1 = Fv[(v1 * kZPairs + pr) * N + m], f2 = Fv[(v2 * kZPairs + pr) * N + m];
+            const double2 f1 = Fv[(v1 * kZPairs + pr) * LZ + m], f2 = Fv[(v2 * kZPairs + pr) * LZ + m];
             pa = f1.x * f2.x;
             pb = f1.y * f2.y;
           }
@@ -758,11 +749,11 @@ __global__ void __launch_bounds__(kThreadsZF, z_min_blocks(NF, FB)) k_z_fused(Di
           if (zsel >= 0 && z != zsel) continue;
           double pa, pb;
           if (fa < 0 || fb < 0) {
-            const double2 f1 = Fv[((fa < 0 ? fb : fa) * kZPairs + pr) * N + m];
+            const double2 f1 = Fv[((fa < 0 ? fb : fa) * kZPairs + pr) * LZ + m];
             pa = f1.x;
             pb = f1.y;
           } else {
-            const double2 f1 = Fv[(fa * kZPairs + pr) * N + m], f2 = Fv[(fb * kZPairs + pr) * N + m];
+            const double2 f1 = Fv[(fa * kZPairs + pr) * LZ + m], f2 = Fv[(fb * kZPairs + pr) * LZ + m];
             pa = f1.x * f2.x;
             pb = f1.y * f2.y;
           }
@@ -790,17 +781,17 @@ __global__ void __launch_bounds__(kThreadsZF, z_min_blocks(NF, FB)) k_z_fused(Di
       const int v1 = qv[0][qg], v2 = qv[1][qg];
       double pa, pb;
       if (v1 < 0 || v2 < 0) {
-        const double2 f1 = Fv[((v1 < 0 ? v2 : v1) * kZPairs + pr) * N + m];
+        const double2 f1 = Fv[((v1 < 0 ? v2 : v1) * kZPairs + pr) * LZ + m];
         pa = f1.x;
         pb = f1.y;
       } else {
-        const double2 f1 = Fv[(v1 * kZPairs + pr) * N + m], f2 = Fv[(v2 * kZPairs + pr) * N + m];
+        const double2 f1 = Fv[(v1 * kZPairs + pr) * LZ + m], f2 = Fv[(v2 * kZPairs + pr) * LZ + m];
         pa = f1.x * f2.x;
         pb = f1.y * f2.y;
       }
       return make_double2(pa, pb);
     };
-    const double2* R = fft_lines_ld<NF, false, NT, FB, false, kPlanHot, kTwl>(A, B, nc, N, pzl, ld);
+    const double2* R = fft_lines_ld<NF, false, NT, FB, false, kPlanHot>(A, B, nc, LZ, pzl, ld);
     // coefficient n of the two packed columns from Z = R[n] and conj(R[N - n]);
     // coefficients n and N - n share those two loads: items n = 0 .. N/2 write
     // n (< NZ) and, for 0 < n < N/2, N - n when it is < NZ
@@ -809,7 +800,7 @@ __global__ void __launch_bounds__(kThreadsZF, z_min_blocks(NF, FB)) k_z_fused(Di
       const int li = idx / NH, n = idx - li * NH;
       const int lg = l0 + li, qg = lg / kZPairs, pr = lg - qg * kZPairs;
       const int n2 = (n == 0) ? 0 : N - n;
-      const double2 Z = R[li * N + n], W = R[li * N + n2];
+      const double2 Z = R[li * LZ + n], W = R[li * LZ + n2];
       double* dst = Q2 + qg * vstride + col0 + (size_t)(2 * pr) * NZ;
       const bool oa = col_ok(2 * pr), ob = col_ok(2 * pr + 1);
       auto out = [&](int k, double2 P, double2 Pm) {  // coefficient k from R[k] = P, R[N - k] = Pm
@@ -836,7 +827,7 @@ __global__ void __launch_bounds__(kThreadsX, hot_min_blocks(kThreadsX)) k_fwd_x(
                                                                                int y0) {
   extern __shared__ double2 sm[];
   const int qi = blockIdx.x, n0 = blockIdx.y * kNB2, y = y0 + blockIdx.z;
-  const int NXA = NF ? NF : d.NXA, NP = kNB2 / 2, LS = NXA + kPadXY;
+  const int NXA = NF ? NF : d.NXA, NP = kNB2 / 2, LS = NF ? line_stride(NF, PV) : NXA + kPadRt;
   double2* A = sm;
   double2* B = sm + NP * LS;  // runtime plan only
   // rows na, na+1 of column x packed as one complex value, produced inside the
@@ -875,7 +866,7 @@ __global__ void __launch_bounds__(kThreadsY, kMinBlocksY) k_fwd_y(Dims d, const 
                                                      FftPlan py) {
   extern __shared__ double2 sm[];
   const int qi = blockIdx.x, n0 = blockIdx.y * kNB1, kx = blockIdx.z;
-  const int NYA = NF ? NF : d.NYA, LS = NYA + kPadY;
+  const int NYA = NF ? NF : d.NYA, LS = NF ? line_stride(NF, kPlanY) : NYA + kPadRt;
   double2* A = sm;
   double2* B = sm + kNB1 * LS;  // runtime plan only
   // produced inside the first FFT pass
@@ -906,7 +897,7 @@ __global__ void __launch_bounds__(kThreadsYF, kMinBlocksYF) k_fwd_y_pipe(Dims d,
   extern __shared__ double2 sm[];
   constexpr int NYA = NF;
   constexpr PlanR P = plan_of(NF, kPlanYF);
-  const int LS = NYA + kPadY;
+  constexpr int LS = line_stride(NF, kPlanYF);
   double2* A = sm;                 // kNB1 lines, stride LS
   double2* stg = A + kNB1 * LS;    // staged input [y][kNB1]
   const int nnb = (d.NZ + kNB1 - 1) / kNB1;
@@ -933,9 +924,9 @@ __global__ void __launch_bounds__(kThreadsYF, kMinBlocksYF) k_fwd_y_pipe(Dims d,
       const double2 v = stg[y * kNB1 + ln];
       return (n0 + ln == 0) ? cscale(v, 0.5) : v;
     };
-    fft_pass_first<NF, P.r[0], false, kThreadsYF, kNB1, true>(A, kNB1, LS, ld);  // ends with a barrier
+    fft_pass_first<NF, P.r[0], false, kThreadsYF, kNB1, true, kPlanYF>(A, kNB1, LS, ld);  // ends with a barrier
     issue(tile + gridDim.x);
-    fft_passes<NF, 1, P.r[0], false, kThreadsYF, kNB1, kPlanYF>(A, kNB1, LS, py.tw);
+    fft_passes<NF, 1, P.r[0], false, kThreadsYF, kNB1, kPlanYF, pad_every(NF, kPlanYF, true)>(A, kNB1, LS, py.tws[kPlanYF]);
     // two adjacent Chebyshev rows per thread: one 32-byte store
     for (int idx = threadIdx.x; idx < (kNB1 / 2) * NYA; idx += blockDim.x) {
       const int l0 = 2 * (idx % (kNB1 / 2)), ky = idx / (kNB1 / 2), n = n0 + l0;
@@ -3134,7 +3125,7 @@ template <int NF>
 struct InvY {
   static void run(const Dims& d, int nf, const FullVarDev* fv, StateSet st, const double2* plain_spec,
                   const double* kx, const double* ky, double2* Y1, const FftPlan& py, int single, cudaStream_t s) {
-    size_t sm = (NF ? 1 : 2) * kNB1 * (size_t)(d.NYA + kPadY) * sizeof(double2);
+    size_t sm = (NF ? 1 : 2) * kNB1 * (size_t)(NF ? line_stride(NF, kPlanY) : d.NYA + kPadRt) * sizeof(double2);
     dim3 g(nf, (d.NZ + kNB1 - 1) / kNB1, d.NXH);
     if (single && !plain_spec) {
       set_smem(k_inv_y1<NF>, sm);
@@ -3154,7 +3145,7 @@ struct InvX {
   template <int PV>
   static void go(const Dims& d, int nf, const double2* Y1, double* Y2, const FftPlan& px, int y0, int ny,
                  cudaStream_t s) {
-    size_t sm = (NF ? 1 : 2) * (kNB2 / 2) * (size_t)(d.NXA + kPadXY) * sizeof(double2);
+    size_t sm = (NF ? 1 : 2) * (kNB2 / 2) * (size_t)(NF ? line_stride(NF, PV) : d.NXA + kPadRt) * sizeof(double2);
     set_smem(k_inv_x<NF, PV>, sm);
     dim3 g(nf, (d.NZ + kNB2 - 1) / kNB2, ny);
     k_inv_x<NF, PV><<<g, kThreadsX, sm, s>>>(d, Y1, Y2, px, y0);
@@ -3166,10 +3157,10 @@ struct InvX {
   }
   static void run(const Dims& d, int nf, const double2* Y1, double* Y2, const FftPlan& px, int pv, int tiles,
                   cudaStream_t s) {
-    if constexpr (NF != 0 && tw_pass2_len<NF, 1>() > 0) {
+    if constexpr (NF != 0 && plan_of(NF, 1).nst == 2) {
       if (pv && !tiles) {
         // persistent pipelined kernel: as many CTAs as fit on the device at once
-        const size_t sm = ((kNB2 / 2) * (size_t)(NF + kPadXY) + (size_t)d.NXH * kStgX) * sizeof(double2);
+        const size_t sm = ((kNB2 / 2) * (size_t)line_stride(NF, 1) + (size_t)d.NXH * kStgX) * sizeof(double2);
         set_smem(k_inv_x_pipe<NF>, sm);
         static int nct = 0;
         if (!nct) nct = persistent_ctas(k_inv_x_pipe<NF>, kThreadsXP, sm);
@@ -3209,7 +3200,7 @@ struct ZFused {
                  const double2* dct_tw, const double* wz, const double* wzinv, unsigned long long* cfl_bits,
                  double* ke_partial, int y0, int ny, cudaStream_t s) {
     const size_t lines = (size_t)nf * kZPairs + FB + (NF ? 0 : std::max(kZLines, FB));
-    const size_t sm = lines * d.NZA * sizeof(double2);
+    const size_t sm = lines * (NF ? line_len(NF, kPlanHot, false) : d.NZA) * sizeof(double2);
     set_smem(k_z_fused<NF, FB>, sm);
     dim3 g((d.NXA + 2 * kZPairs - 1) / (2 * kZPairs), ny);
     k_z_fused<NF, FB><<<g, z_threads_fused(NF, FB), sm, s>>>(d, nf, q, Y2, Q2, pz, dct_tw, wz, wzinv, cfl_bits,
@@ -3231,7 +3222,7 @@ struct FwdX {
   template <int PV>
   static void go(const Dims& d, int nq, const double* Q2, double2* Q1, const FftPlan& px, int y0, int ny,
                  cudaStream_t s) {
-    size_t sm = (NF ? 1 : 2) * (kNB2 / 2) * (size_t)(d.NXA + kPadXY) * sizeof(double2);
+    size_t sm = (NF ? 1 : 2) * (kNB2 / 2) * (size_t)(NF ? line_stride(NF, PV) : d.NXA + kPadRt) * sizeof(double2);
     set_smem(k_fwd_x<NF, PV>, sm);
     dim3 g(nq, (d.NZ + kNB2 - 1) / kNB2, ny);
     k_fwd_x<NF, PV><<<g, kThreadsX, sm, s>>>(d, Q2, Q1, px, y0);
@@ -3249,7 +3240,7 @@ struct FwdY {
     if constexpr (NF != 0) {
       if (!grid_variant) {
       // persistent pipelined kernel: as many CTAs as fit on the device at once
-      const size_t sm = (kNB1 * (size_t)(NF + kPadY) + (size_t)NF * kNB1) * sizeof(double2);
+      const size_t sm = (kNB1 * (size_t)line_stride(NF, kPlanYF) + (size_t)NF * kNB1) * sizeof(double2);
       set_smem(k_fwd_y_pipe<NF>, sm);
       static int nct = 0;
       if (!nct) nct = persistent_ctas(k_fwd_y_pipe<NF>, kThreadsYF, sm);
@@ -3258,7 +3249,7 @@ struct FwdY {
       return;
     }
     }
-    size_t sm = (NF ? 1 : 2) * kNB1 * (size_t)(d.NYA + kPadY) * sizeof(double2);
+    size_t sm = (NF ? 1 : 2) * kNB1 * (size_t)(NF ? line_stride(NF, kPlanY) : d.NYA + kPadRt) * sizeof(double2);
     set_smem(k_fwd_y<NF>, sm);
     dim3 g(nq, (d.NZ + kNB1 - 1) / kNB1, d.NXH);
     k_fwd_y<NF><<<g, kThreadsY, sm, s>>>(d, Q1, qspec, scale, py);

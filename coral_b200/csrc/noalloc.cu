@@ -21,8 +21,11 @@ using namespace coral;
 namespace {
 
 constexpr size_t kScratchBytes = size_t(64) << 20;  // 64 MiB, the stated maximum
+constexpr int kMaxTableLen = 4096;                  // 6 tables of < 2 N entries fit kTableBytes
 constexpr int kMaxModes = 1 << 16;                  // per direction, checked first
-__device__ __align__(256) unsigned char g_scratch[kScratchBytes];
+// beyond the stated maximum: the pass tables of the compiled FFT plans (two per axis)
+constexpr size_t kTableBytes = size_t(1) << 20;
+__device__ __align__(256) unsigned char g_scratch[kScratchBytes + kTableBytes];
 
 // The device address of g_scratch, looked up once per device and CUDA context
 // with that device current (in host code the array's name is only a stand-in
@@ -88,14 +91,31 @@ void* scratch_address() {
   return slot.addr;
 }
 
-// exp(-i pi k * f / N) for k < N, from sincospi: f = 2 gives the FFT twiddles,
-// f = 1/2 the pre/post-rotation of the FFT-based Chebyshev transform
-__global__ void k_twiddles(double2* tw, int N, double f) {
-  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < N; k += gridDim.x * blockDim.x) {
-    double s, c;
-    sincospi(-f * (double)k / (double)N, &s, &c);
-    tw[k] = make_double2(c, s);
+// The twiddle tables of a call in one launch: per axis exp(-2 pi i k / N), k < N,
+// and the pass tables of the compiled plans (entries of the former); for z also
+// exp(-i pi k / 2N), the rotation of the FFT-based Chebyshev transform
+struct Tables {
+  int N[3];
+  double2* tw[3];
+  double2* tws[3][2];
+  int len[3][2];
+  double2* dct;
+};
+__device__ __forceinline__ double2 unit_root(double a, int N) {  // exp(-i pi a / N)
+  double s, c;
+  sincospi(-a / (double)N, &s, &c);
+  return make_double2(c, s);
+}
+__global__ void k_twiddles(Tables t) {
+  const int i0 = blockIdx.x * blockDim.x + threadIdx.x, st = gridDim.x * blockDim.x;
+  for (int ax = 0; ax < 3; ++ax) {
+    const int N = t.N[ax];
+    for (int k = i0; k < N; k += st) t.tw[ax][k] = unit_root(2.0 * (double)k, N);
+    for (int pv = 0; pv < 2; ++pv)
+      for (int i = i0; i < t.len[ax][pv]; i += st)
+        t.tws[ax][pv][i] = unit_root(2.0 * (double)pass_tw_index(N, pv, i), N);
   }
+  for (int k = i0; k < t.N[2]; k += st) t.dct[k] = unit_root(0.5 * (double)k, t.N[2]);
 }
 
 bool smooth23(int n) {
@@ -160,12 +180,19 @@ extern "C" int coral_spec_to_phys_noalloc(int NX, int NY, int NZ, const double* 
     double* Y2 = reinterpret_cast<double*>(base + o_y2);
     // every scratch byte that is read is written first in this call (twiddles,
     // then the y pass fills Y1, the x pass fills Y2), so nothing needs clearing
-    k_twiddles<<<8, 128, 0, s>>>(ty, NYA, 2.0);
-    k_twiddles<<<8, 128, 0, s>>>(tx, NXA, 2.0);
-    k_twiddles<<<8, 128, 0, s>>>(tz, NZA, 2.0);
-    k_twiddles<<<8, 128, 0, s>>>(td, NZA, 0.5);
     const Dims d{NXH, NYA, NXA, NZ, NZA};
-    const FftPlan py = plan_in(NYA, ty), px = plan_in(NXA, tx), pz = plan_in(NZA, tz);
+    FftPlan pl[3] = {plan_in(NYA, ty), plan_in(NXA, tx), plan_in(NZA, tz)};
+    Tables tab{{NYA, NXA, NZA}, {ty, tx, tz}, {}, {}, td};
+    size_t at = kScratchBytes;
+    for (int ax = 0; ax < 3; ++ax)
+      for (int pv = 0; pv < 2; ++pv) {
+        // (axes longer than the compiled lengths take run-time plans, no pass tables)
+        tab.len[ax][pv] = tab.N[ax] <= kMaxTableLen ? pass_tw_len(tab.N[ax], pv) : 0;
+        pl[ax].tws[pv] = tab.tws[ax][pv] = reinterpret_cast<double2*>(base + at);
+        at += up256((size_t)tab.len[ax][pv] * sizeof(double2));
+      }
+    k_twiddles<<<16, 128, 0, s>>>(tab);
+    const FftPlan &py = pl[0], &px = pl[1], &pz = pl[2];
     launch_inv_y(d, 1, nullptr, StateSet{}, reinterpret_cast<const double2*>(spec), nullptr, nullptr, Y1, py, s);
     launch_inv_x(d, 1, Y1, Y2, px, s);
     launch_inv_z(d, 1, Y2, phys, pz, td, nullptr, nullptr, s);

@@ -113,11 +113,30 @@ __device__ double2* fft_lines(double2* A, double2* B, int nl, int LS, const FftP
 // waits for every thread to have loaded (so the pass can write in place), and
 // stores its R outputs at their Stockham (self-sorting) positions.  Only one
 // line buffer is needed.
+// A plan is a list of passes; an entry r < 100 is one radix, a 100 + b (or
+// (a 100 + b) 100 + c) a pass that takes the radices a, b (, c) one after the other
+// in registers, with the arithmetic of separate passes bit for bit (the solves
+// turn another rounding of the transforms into 1e-9 of the pressure, so a length
+// keeps its radices when its passes are merged).
 struct PlanR {
   int nst;
   int r[12];
 };
+__host__ __device__ constexpr int radix_a(int code) { return code < 100 ? code : code < 10000 ? code / 100 : code / 10000; }
+__host__ __device__ constexpr int radix_b(int code) { return code < 100 ? 1 : code < 10000 ? code % 100 : code / 100 % 100; }
+__host__ __device__ constexpr int radix_c(int code) { return code < 10000 ? 1 : code % 100; }
+__host__ __device__ constexpr int radix_of(int code) { return radix_a(code) * radix_b(code) * radix_c(code); }
 __host__ __device__ constexpr PlanR make_planr(int N) {
+  switch (N) {
+    case 54: return PlanR{2, {303, 302}};
+    case 108: return PlanR{2, {403, 303}};
+    case 162: return PlanR{2, {303, 30302}};
+    case 216: return PlanR{2, {403, 30302}};
+    case 324: return PlanR{2, {403, 30303}};
+    case 432: return PlanR{2, {404, 30303}};
+    case 486: return PlanR{3, {303, 303, 302}};
+    default: break;
+  }
   PlanR p{0, {}};
   int n = N, a = 0, b = 0;
   while (n % 3 == 0) { n /= 3; ++b; }
@@ -316,21 +335,31 @@ __device__ __forceinline__ void dft(double2 (&x)[R]) {
   }
 }
 
-// Twiddles of the passes S >= 1 of a compiled plan, one table [r - 1][k] after the
-// other: entry (r, k), 1 <= r < R, k < Ns (the product of the earlier radices), is
-// exp(-2 pi i r k / (Ns R)).  Consecutive lanes take consecutive k, so a load touches
-// consecutive 16-byte words (the N-entry table read at stride r touched up to a
-// line per lane).  With the padding below, per step at 384^2 x 192: inverse y
-// 2.91 -> 2.48 ms, inverse x 2.38 -> 2.20, forward x 3.48 -> 3.16, forward y 3.59
-// -> 3.38, z 9.3 -> 9.07; z at 96 points 0.54 -> 0.46 ms.
+// Twiddles of a compiled plan's radices in their order (those of merged passes one by
+// one) after the first, one table [r - 1][k] after the other: entry (r, k),
+// 1 <= r < R, k < Ns (the product of the earlier radices), is exp(-2 pi i r k / (Ns R)).
+// Consecutive lanes take consecutive k, so a load touches consecutive 16-byte words
+// (the N-entry table read at stride r touched up to a line per lane).  With the
+// padding below, per step at 384^2 x 192: inverse y 2.91 -> 2.48 ms, inverse x 2.38
+// -> 2.20, forward x 3.48 -> 3.16, forward y 3.59 -> 3.38, z 9.3 -> 9.07; z at 96
+// points 0.54 -> 0.46 ms.
 __host__ __device__ constexpr int pass_ns(int N, int PV, int S) {
   int ns = 1;
-  for (int q = 0; q < S; ++q) ns *= plan_of(N, PV).r[q];
+  for (int q = 0; q < S; ++q) ns *= radix_of(plan_of(N, PV).r[q]);
   return ns;
 }
-__host__ __device__ constexpr int pass_tw_offset(int N, int PV, int S) {
-  int o = 0;
-  for (int q = 1; q < S; ++q) o += pass_ns(N, PV, q) * (plan_of(N, PV).r[q] - 1);
+// entries of the tables before radix q (0, 1, 2) of pass S
+__host__ __device__ constexpr int pass_tw_offset(int N, int PV, int S, int q = 0) {
+  const PlanR p = plan_of(N, PV);
+  int o = 0, ns = 1;
+  for (int t = 0; t <= S && t < p.nst; ++t) {
+    const int r[3] = {radix_a(p.r[t]), radix_b(p.r[t]), radix_c(p.r[t])};
+    for (int u = 0; u < 3; ++u) {
+      if (t == S && u == q) return o;
+      if (ns > 1) o += ns * (r[u] - 1);
+      ns *= r[u];
+    }
+  }
   return o;
 }
 __host__ __device__ constexpr int pass_tw_len(int N, int PV) { return pass_tw_offset(N, PV, plan_of(N, PV).nst); }
@@ -338,11 +367,14 @@ __host__ __device__ constexpr int pass_tw_len(int N, int PV) { return pass_tw_of
 __host__ __device__ inline int pass_tw_index(int N, int PV, int i) {
   const PlanR p = plan_of(N, PV);
   int ns = 1;
-  for (int s = 0; s < p.nst; ++s) {
-    const int n = s == 0 ? 0 : ns * (p.r[s] - 1);
-    if (i < n) return (i / ns + 1) * (i % ns) * (N / (ns * p.r[s]));
-    i -= n;
-    ns *= p.r[s];
+  for (int t = 0; t < p.nst; ++t) {
+    const int r[3] = {radix_a(p.r[t]), radix_b(p.r[t]), radix_c(p.r[t])};
+    for (int u = 0; u < 3; ++u) {
+      const int n = ns > 1 ? ns * (r[u] - 1) : 0;
+      if (i < n) return (i / ns + 1) * (i % ns) * (N / (ns * r[u]));
+      i -= n;
+      ns *= r[u];
+    }
   }
   return 0;
 }
@@ -354,13 +386,14 @@ __host__ __device__ inline int pass_tw_index(int N, int PV, int i) {
 // butterflies).  Odd radices need none, and later passes store in natural order.
 __host__ __device__ constexpr int pad_every(int N, int PV, bool line_fast) {
   const PlanR p = plan_of(N, PV);
-  if (p.nst != 2 || p.r[0] % 2) return 0;
+  const int r0 = radix_of(p.r[0]);
+  if (p.nst != 2 || r0 % 2) return 0;
   if (line_fast) return 1;
-  return p.r[0] % 8 == 0 ? 1 : p.r[0] % 4 == 0 ? 2 : 4;
+  return r0 % 8 == 0 ? 1 : r0 % 4 == 0 ? 2 : 4;
 }
 __host__ __device__ constexpr int line_len(int N, int PV, bool line_fast) {
   const int e = N ? pad_every(N, PV, line_fast) : 0;
-  return e ? N + (N / plan_of(N, PV).r[0] - 1) / e : N;
+  return e ? N + (N / radix_of(plan_of(N, PV).r[0]) - 1) / e : N;
 }
 // line stride of the passes that walk 4 interleaved lines: 2 mod 8, so that the
 // same position of the lines hits 4 distinct even 16-byte bank groups
@@ -369,11 +402,81 @@ __host__ __device__ constexpr int line_stride(int N, int PV) {
   return n == N ? N + 2 : (n + 5) / 8 * 8 + 2;
 }
 
-// One in-place pass of radix R over nl lines (line stride LS) by NT threads;
-// NLMAX bounds nl (registers hold ceil(NLMAX N / (R NT)) butterflies per thread);
-// tw: the pass's table; PADE: pad_every of the line as the first pass left it.
-template <int N, int R, int Ns, bool INV, int NT, int NLMAX, int PADE = 0>
+// The radices of a merged pass S in registers: x[r] is the element at position j + r N / R of
+// the line, k = j mod Ns.  Radix a combines x[r' + r1 (R / a)] over r1 for every r',
+// radix b then the results over the next digit, and so on; the twiddle of digit r_b
+// has k + r_a Ns in place of k, and the outputs come in order.  tw: the plan's
+// tables (null only when no twiddle is needed).
+template <int N, int PV, int S, bool INV, int R>
+__device__ __forceinline__ void pass_butterfly(double2 (&x)[R], int k, const double2* __restrict__ tw) {
+  constexpr int code = plan_of(N, PV).r[S], Ra = radix_a(code), Rb = radix_b(code), Rc = radix_c(code);
+  constexpr int Ns = pass_ns(N, PV, S);
+  static_assert(R == Ra * Rb * Rc, "radix");
+  auto twiddle = [&](double2 v, int at) {
+    double2 w = tw[at];
+    if (INV) w = cconj(w);
+    return cmul(v, w);
+  };
+  constexpr int M = Rb * Rc;
+  double2 y[R];  // y[ra M + r']
+#pragma unroll
+  for (int q = 0; q < M; ++q) {
+    double2 v[Ra];
+#pragma unroll
+    for (int r = 0; r < Ra; ++r) {
+      v[r] = x[q + r * M];
+      if (Ns > 1 && r > 0) v[r] = twiddle(v[r], pass_tw_offset(N, PV, S) + (r - 1) * Ns + k);
+    }
+    dft<Ra, INV>(v);
+#pragma unroll
+    for (int r = 0; r < Ra; ++r) y[r * M + q] = v[r];
+  }
+  // digit rb of r' = rb Rc + rc
+#pragma unroll
+  for (int ra = 0; ra < Ra; ++ra)
+#pragma unroll
+    for (int rc = 0; rc < Rc; ++rc) {
+      double2 v[Rb];
+#pragma unroll
+      for (int r = 0; r < Rb; ++r) {
+        v[r] = y[ra * M + r * Rc + rc];
+        if (r > 0 && Ns * Ra > 1)
+          v[r] = twiddle(v[r], pass_tw_offset(N, PV, S, 1) + (r - 1) * Ns * Ra + k + ra * Ns);
+      }
+      dft<Rb, INV>(v);
+#pragma unroll
+      for (int r = 0; r < Rb; ++r) y[ra * M + r * Rc + rc] = v[r];
+    }
+  if constexpr (Rc > 1) {
+#pragma unroll
+    for (int ra = 0; ra < Ra; ++ra)
+#pragma unroll
+      for (int rb = 0; rb < Rb; ++rb) {
+        double2 v[Rc];
+#pragma unroll
+        for (int r = 0; r < Rc; ++r) {
+          v[r] = y[ra * M + rb * Rc + r];
+          if (r > 0) v[r] = twiddle(v[r], pass_tw_offset(N, PV, S, 2) + (r - 1) * Ns * Ra * Rb + k + (ra + rb * Ra) * Ns);
+        }
+        dft<Rc, INV>(v);
+#pragma unroll
+        for (int r = 0; r < Rc; ++r) y[ra * M + rb * Rc + r] = v[r];
+      }
+  }
+#pragma unroll
+  for (int ra = 0; ra < Ra; ++ra)
+#pragma unroll
+    for (int rb = 0; rb < Rb; ++rb)
+#pragma unroll
+      for (int rc = 0; rc < Rc; ++rc) x[ra + Ra * (rb + Rb * rc)] = y[ra * M + rb * Rc + rc];
+}
+
+// Pass S in place over nl lines (line stride LS) by NT threads; NLMAX bounds nl
+// (registers hold ceil(NLMAX N / (R NT)) butterflies per thread); tw: the plan's
+// tables; PADE: pad_every of the line as the first pass left it.
+template <int N, int PV, int S, bool INV, int NT, int NLMAX, int PADE = 0>
 __device__ __forceinline__ void fft_pass(double2* A, int nl, int LS, const double2* __restrict__ tw) {
+  constexpr int R = radix_of(plan_of(N, PV).r[S]), Ns = pass_ns(N, PV, S);
   constexpr int NB = N / R;               // butterflies per line
   static_assert(PADE == 0 || NB == Ns, "padding: second of two passes");
   constexpr int BPT = (NLMAX * NB + NT - 1) / NT;
@@ -387,16 +490,21 @@ __device__ __forceinline__ void fft_pass(double2* A, int nl, int LS, const doubl
       const double2* sl = A + line * LS + j;
 #pragma unroll
       for (int r = 0; r < R; ++r) v[i][r] = sl[r * NB + (PADE ? r / PADE : 0)];
-      if constexpr (Ns > 1) {
-        const int k = j % Ns;
+      if constexpr (plan_of(N, PV).r[S] >= 100) {
+        pass_butterfly<N, PV, S, INV>(v[i], j % Ns, tw);
+      } else {
+        if constexpr (Ns > 1) {
+          const int k = j % Ns;
+          const double2* tp = tw + pass_tw_offset(N, PV, S);
 #pragma unroll
-        for (int r = 1; r < R; ++r) {
-          double2 w = tw[(r - 1) * Ns + k];
-          if (INV) w = cconj(w);
-          v[i][r] = cmul(v[i][r], w);
+          for (int r = 1; r < R; ++r) {
+            double2 w = tp[(r - 1) * Ns + k];
+            if (INV) w = cconj(w);
+            v[i][r] = cmul(v[i][r], w);
+          }
         }
+        dft<R, INV>(v[i]);
       }
-      dft<R, INV>(v[i]);
     }
   }
   __syncthreads();
@@ -413,15 +521,15 @@ __device__ __forceinline__ void fft_pass(double2* A, int nl, int LS, const doubl
   __syncthreads();
 }
 
-// The first pass (Ns = 1, no twiddles) with its inputs produced by ld(line, k)
-// (k = position in the line) instead of read from shared memory; it writes its
-// outputs in place into A, which nothing reads during the pass, so it needs no
-// barrier between loads and stores.
+// The first pass with its inputs produced by ld(line, k) (k = position in the line)
+// instead of read from shared memory; it writes its outputs in place into A, which
+// nothing reads during the pass, so it needs no barrier between loads and stores.
 // LINE_FAST: consecutive threads take consecutive lines at the same position
 // (so that interleaved lines of a global array load together); otherwise
 // consecutive positions of one line.
-template <int N, int R, bool INV, int NT, int NLMAX, bool LINE_FAST, int PV, class Load>
-__device__ __forceinline__ void fft_pass_first(double2* A, int nl, int LS, Load&& ld) {
+template <int N, bool INV, int NT, int NLMAX, bool LINE_FAST, int PV, class Load>
+__device__ __forceinline__ void fft_pass_first(double2* A, int nl, int LS, const double2* __restrict__ tw, Load&& ld) {
+  constexpr int R = radix_of(plan_of(N, PV).r[0]);
   constexpr int NB = N / R, PADE = pad_every(N, PV, LINE_FAST);
   constexpr int BPT = (NLMAX * NB + NT - 1) / NT;
   const int total = nl * NB;
@@ -434,7 +542,8 @@ __device__ __forceinline__ void fft_pass_first(double2* A, int nl, int LS, Load&
       double2 v[R];
 #pragma unroll
       for (int r = 0; r < R; ++r) v[r] = ld(line, j + r * NB);
-      dft<R, INV>(v);
+      if constexpr (plan_of(N, PV).r[0] >= 100) pass_butterfly<N, PV, 0, INV>(v, 0, tw);
+      else dft<R, INV>(v);
       double2* dl = A + line * LS + j * R + (PADE ? j / PADE : 0);
 #pragma unroll
       for (int r = 0; r < R; ++r) dl[r] = v[r];
@@ -443,15 +552,13 @@ __device__ __forceinline__ void fft_pass_first(double2* A, int nl, int LS, Load&
   __syncthreads();
 }
 
-// passes S, S + 1, ... of plan variant PV; tw: the plan's pass tables; PADE as
+// passes S, S + 1, ... of plan variant PV; tw: the plan's tables; PADE as
 // fft_pass's (of pass 1)
-template <int N, int S, int Ns, bool INV, int NT, int NLMAX, int PV = 0, int PADE = 0>
+template <int N, int S, bool INV, int NT, int NLMAX, int PV = 0, int PADE = 0>
 __device__ __forceinline__ void fft_passes(double2* A, int nl, int LS, const double2* tw) {
-  constexpr PlanR P = plan_of(N, PV);
-  if constexpr (S < P.nst) {
-    constexpr int R = P.r[S];
-    fft_pass<N, R, Ns, INV, NT, NLMAX, S == 1 ? PADE : 0>(A, nl, LS, tw + pass_tw_offset(N, PV, S));
-    fft_passes<N, S + 1, Ns * R, INV, NT, NLMAX, PV, PADE>(A, nl, LS, tw);
+  if constexpr (S < plan_of(N, PV).nst) {
+    fft_pass<N, PV, S, INV, NT, NLMAX, S == 1 ? PADE : 0>(A, nl, LS, tw);
+    fft_passes<N, S + 1, INV, NT, NLMAX, PV, PADE>(A, nl, LS, tw);
   }
 }
 
@@ -472,10 +579,9 @@ __device__ __forceinline__ double2* fft_lines_ld(double2* A, double2* B, int nl,
     __syncthreads();
     return fft_lines<INV>(A, B, nl, LS, p);
   } else {
-    constexpr PlanR P = plan_of(NC, PV);
-    static_assert(P.nst > 0, "transform length must be 2^a 3^b");
-    fft_pass_first<NC, P.r[0], INV, NT, NLMAX, LINE_FAST, PV>(A, nl, LS, ld);
-    fft_passes<NC, 1, P.r[0], INV, NT, NLMAX, PV, pad_every(NC, PV, LINE_FAST)>(A, nl, LS, p.tws[PV]);
+    static_assert(plan_of(NC, PV).nst > 0, "transform length must be 2^a 3^b");
+    fft_pass_first<NC, INV, NT, NLMAX, LINE_FAST, PV>(A, nl, LS, p.tws[PV], ld);
+    fft_passes<NC, 1, INV, NT, NLMAX, PV, pad_every(NC, PV, LINE_FAST)>(A, nl, LS, p.tws[PV]);
     return A;
   }
 }
@@ -487,7 +593,7 @@ __device__ __forceinline__ double2* fft_lines_n(double2* A, double2* B, int nl, 
     return fft_lines<INV>(A, B, nl, LS, p);
   } else {
     static_assert(make_planr(NC).nst > 0, "transform length must be 2^a 3^b");
-    fft_passes<NC, 0, 1, INV, NT, NLMAX>(A, nl, LS, p.tws[0]);
+    fft_passes<NC, 0, INV, NT, NLMAX>(A, nl, LS, p.tws[0]);
     return A;
   }
 }

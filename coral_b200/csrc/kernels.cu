@@ -39,13 +39,18 @@ constexpr int kThreads = 256;
 constexpr int kPlanHot = 1;
 constexpr int kPlanY = 0;
 // x / y passes: threads per CTA for nl lines of a compiled length N, the most
-// butterflies of any pass rounded up to whole warps (one butterfly per thread
-// per pass); 256 for the run-time plans
+// that any pass keeps busy, rounded up to whole warps: one butterfly per thread,
+// of radix 2, 3 and 4 as many as make 8 or 9 elements (one radix-3 butterfly each
+// left the radix-8 passes of 192 = 3 x 8 x 8 with 96 of 256 threads); 256 for the
+// run-time plans
 __host__ __device__ constexpr int xy_threads(int N, int nl, int pv) {
   if (N == 0) return 256;
   const PlanR p = plan_of(N, pv);
   int m = 32;
-  for (int i = 0; i < p.nst; ++i) m = (nl * N / p.r[i] > m) ? nl * N / p.r[i] : m;
+  for (int i = 0; i < p.nst; ++i) {
+    const int r = radix_of(p.r[i]), per = r <= 4 ? 9 / r : 1, t = (nl * N / r + per - 1) / per;
+    m = t > m ? t : m;
+  }
   return (m + 31) / 32 * 32;
 }
 #define kThreadsX xy_threads(NF, kNB2 / 2, PV)
@@ -58,9 +63,11 @@ constexpr int kPlanYF = 1;
 // CTAs per SM the kernels with two-pass plans are compiled for: registers
 // capped at no fewer than 128 per thread
 __host__ __device__ constexpr int hot_min_blocks(int nt) { return 65536 / (nt * 128) > 1 ? 65536 / (nt * 128) : 1; }
-// CTAs per SM of the y passes (measured best at 384^2 x 192) and of the
-// separate z passes of the transform API paths
-constexpr int kMinBlocksY = 3;
+// CTAs per SM of the y passes: 3, measured best at 384^2 x 192; fewer where that
+// would leave a thread under 64 registers
+__host__ __device__ constexpr int y_min_blocks(int nt) { return 65536 / (nt * 64) < 3 ? 65536 / (nt * 64) : 3; }
+#define kMinBlocksY y_min_blocks(kThreadsY)
+// CTAs per SM of the separate forward z pass
 constexpr int kMinBlocksZ = 4;
 constexpr int kWPB = 8;  // warps (systems) per CTA in the per-system kernels
 
@@ -377,9 +384,9 @@ __global__ void __launch_bounds__(kThreadsXP, 3) k_inv_x_pipe(Dims d, int nf, co
       if (p == 0) return make_double2(a.x, b.x);
       return lo ? make_double2(a.x - b.y, a.y + b.x) : make_double2(a.x + b.y, b.x - a.y);
     };
-    fft_pass_first<NF, P.r[0], true, NT, NP, true, 1>(A, NP, LS, ld);  // ends with a barrier
+    fft_pass_first<NF, true, NT, NP, true, 1>(A, NP, LS, s_tw, ld);  // ends with a barrier
     issue(tile + gridDim.x);
-    fft_passes<NF, 1, P.r[0], true, NT, NP, 1, pad_every(NF, 1, true)>(A, NP, LS, s_tw);
+    fft_passes<NF, 1, true, NT, NP, 1, pad_every(NF, 1, true)>(A, NP, LS, s_tw);
     double* dst0 = Y2 + ((size_t)f * d.NYA + y) * NXA * NZ;
     for (int idx = threadIdx.x; idx < NP * NXA; idx += NT) {
       const int m = idx % NP, x = idx / NP, na = n0 + 2 * m;
@@ -401,49 +408,60 @@ __device__ __forceinline__ void atomic_max_nonneg(unsigned long long* addr, doub
   atomicMax(addr, (unsigned long long)__double_as_longlong(v));
 }
 
+// Threads of the z kernels for nl lines of a compiled length N: enough for
+// one butterfly per thread in the radix >= 8 passes and two in the radix-2/4
+// passes (N = 288, 8 lines, plan 18 x 16: 160 threads).
+__host__ __device__ constexpr int z_threads(int N, int nl, int pv = kPlanHot) {
+  if (N == 0) return 256;
+  const PlanR p = plan_of(N, pv);
+  int m = 32;
+  for (int i = 0; i < p.nst; ++i) {
+    const int b = nl * N / radix_of(p.r[i]), per = (radix_of(p.r[i]) <= 4) ? (b + 1) / 2 : b;
+    m = per > m ? per : m;
+  }
+  return (m + 31) / 32 * 32;
+}
+
 // ------------------------------------------------------------------------------
 // inverse transform, pass 3: z REDFT01 with zero padding NZ -> NZAA (transforms.f90:216-223)
 // via an NZAA-point complex FFT (two columns per FFT); also the CFL maxima of
 // compute_cfl_based_timestep (marching.f90:219-238) for the first three full variables
 // ------------------------------------------------------------------------------
+#define kThreadsIZ z_threads(NF, kXB3 / 2, kPlanY)
 template <int NF>
-__global__ void __launch_bounds__(kThreads, kMinBlocksZ) k_inv_z(Dims d, const double* Y2, double* phys, FftPlan pz,
-                                                     const double2* dct_tw, const double* wz,
-                                                     unsigned long long* cfl_bits) {
+__global__ void __launch_bounds__(kThreadsIZ, hot_min_blocks(kThreadsIZ)) k_inv_z(Dims d, const double* Y2, double* phys,
+                                                                                 FftPlan pz, const double2* dct_tw,
+                                                                                 const double* wz,
+                                                                                 unsigned long long* cfl_bits) {
+  constexpr int NT = kThreadsIZ;
   extern __shared__ double2 sm[];
-  __shared__ double red[kThreads / 32];
+  __shared__ double red[NT / 32];
   const int f = blockIdx.x, x0 = blockIdx.y * kXB3, y = blockIdx.z;
-  const int N = NF ? NF : d.NZA, NP = kXB3 / 2;
+  const int N = NF ? NF : d.NZA, NP = kXB3 / 2, LZ = NF ? line_len(NF, kPlanY, false) : N;
   double2* A = sm;
-  double2* B = sm + NP * N;
-  for (int idx = threadIdx.x; idx < NP * N; idx += blockDim.x) {
-    const int m = idx / N, n = idx - m * N;
-    const int xa = x0 + 2 * m, xb = xa + 1;
-    const double* sa = Y2 + (((size_t)f * d.NYA + y) * d.NXA + xa) * d.NZ;
+  double2* B = sm + NP * LZ;  // runtime plan only
+  const double* src0 = Y2 + (((size_t)f * d.NYA + y) * d.NXA + x0) * d.NZ;
+  // X_n and X_{N-n} of the pair's columns, twiddled, packed as va + i vb, produced
+  // inside the first FFT pass (as in the fused kernel)
+  auto ld = [&](int m, int n) -> double2 {
+    const double* sa = src0 + (size_t)(2 * m) * d.NZ;
     const double* sb = sa + d.NZ;
-    double a0 = 0, a1 = 0, b0 = 0, b1 = 0;  // X_n, X_{N-n}
-    if (xa < d.NXA) {
-      if (n < d.NZ) a0 = sa[n];
-      if (n > 0 && N - n < d.NZ) a1 = sa[N - n];
-    }
-    if (xb < d.NXA) {
-      if (n < d.NZ) b0 = sb[n];
-      if (n > 0 && N - n < d.NZ) b1 = sb[N - n];
-    }
+    const bool ha = x0 + 2 * m < d.NXA, hb = x0 + 2 * m + 1 < d.NXA, lo = n < d.NZ, hi = n > 0 && N - n < d.NZ;
+    const double a0 = (lo && ha) ? sa[n] : 0.0, a1 = (hi && ha) ? sa[N - n] : 0.0;
+    const double b0 = (lo && hb) ? sb[n] : 0.0, b1 = (hi && hb) ? sb[N - n] : 0.0;
     const double2 w = cconj(dct_tw[n]);  // exp(+i pi n / 2N)
-    double2 va = cmul(w, make_double2(a0, -a1));
-    double2 vb = cmul(w, make_double2(b0, -b1));
-    A[m * N + n] = make_double2(va.x - vb.y, va.y + vb.x);  // va + i vb
-  }
-  __syncthreads();
-  const double2* R = fft_lines_n<NF, true, kThreads, kXB3 / 2>(A, B, NP, N, pz);
+    const double2 va = cmul(w, make_double2(a0, -a1));
+    const double2 vb = cmul(w, make_double2(b0, -b1));
+    return make_double2(va.x - vb.y, va.y + vb.x);
+  };
+  const double2* R = fft_lines_ld<NF, true, NT, kXB3 / 2, false, kPlanY>(A, B, NP, LZ, pz, ld);
   double mx = 0.0;
   const int which = (f < 3) ? f : -1;
   for (int idx = threadIdx.x; idx < NP * N; idx += blockDim.x) {
     const int m = idx / N, k = idx - m * N;
     const int xa = x0 + 2 * m, xb = xa + 1;
     const int zi = (k & 1) ? (N - 1 - (k >> 1)) : (k >> 1);
-    const double2 z = R[m * N + zi];
+    const double2 z = R[m * LZ + zi];
     double* dst = phys + (((size_t)f * d.NYA + y) * d.NXA + xa) * N;
     if (xa < d.NXA) dst[k] = z.x;
     if (xb < d.NXA) dst[N + k] = z.y;
@@ -558,19 +576,6 @@ __global__ void __launch_bounds__(kThreads, kMinBlocksZ) k_fwd_z(Dims d, int nf,
 // takes, so the products are formed position by position.
 // ------------------------------------------------------------------------------
 
-// Threads of the fused z kernel for nl lines of a compiled length N: enough for
-// one butterfly per thread in the radix >= 8 passes and two in the radix-2/4
-// passes (N = 288, 8 lines, plan 18 x 16: 160 threads).
-__host__ __device__ constexpr int z_threads(int N, int nl) {
-  if (N == 0) return 256;
-  const PlanR p = plan_of(N, kPlanHot);
-  int m = 32;
-  for (int i = 0; i < p.nst; ++i) {
-    const int b = nl * N / p.r[i], per = (p.r[i] <= 4) ? (b + 1) / 2 : b;
-    m = per > m ? per : m;
-  }
-  return (m + 31) / 32 * 32;
-}
 constexpr int kZPairs = 2;               // x-column pairs per CTA
 constexpr int kZLines = 4 * kZPairs;     // lines per inverse FFT batch (4 full variables x 2 pairs)
 // lines per forward FFT batch ((quadratic variable, pair) lines), the kernel's
@@ -581,7 +586,8 @@ __host__ __device__ constexpr int z_threads_fused(int N, int fb) {
   return z_threads(N, kZLines) > z_threads(N, fb) ? z_threads(N, kZLines) : z_threads(N, fb);
 }
 __host__ __device__ constexpr int z_min_blocks(int N, int fb) {
-  return fb < kZFwd ? 3 : hot_min_blocks(z_threads_fused(N, fb));
+  const int hot = hot_min_blocks(z_threads_fused(N, fb));
+  return fb < kZFwd && hot > 3 ? 3 : hot;
 }
 #define kThreadsZF z_threads_fused(NF, FB)
 
@@ -896,7 +902,6 @@ __global__ void __launch_bounds__(kThreadsYF, kMinBlocksYF) k_fwd_y_pipe(Dims d,
                                                                         double2* qspec, double scale, FftPlan py) {
   extern __shared__ double2 sm[];
   constexpr int NYA = NF;
-  constexpr PlanR P = plan_of(NF, kPlanYF);
   constexpr int LS = line_stride(NF, kPlanYF);
   double2* A = sm;                 // kNB1 lines, stride LS
   double2* stg = A + kNB1 * LS;    // staged input [y][kNB1]
@@ -924,9 +929,9 @@ __global__ void __launch_bounds__(kThreadsYF, kMinBlocksYF) k_fwd_y_pipe(Dims d,
       const double2 v = stg[y * kNB1 + ln];
       return (n0 + ln == 0) ? cscale(v, 0.5) : v;
     };
-    fft_pass_first<NF, P.r[0], false, kThreadsYF, kNB1, true, kPlanYF>(A, kNB1, LS, ld);  // ends with a barrier
+    fft_pass_first<NF, false, kThreadsYF, kNB1, true, kPlanYF>(A, kNB1, LS, py.tws[kPlanYF], ld);  // ends with a barrier
     issue(tile + gridDim.x);
-    fft_passes<NF, 1, P.r[0], false, kThreadsYF, kNB1, kPlanYF, pad_every(NF, kPlanYF, true)>(A, kNB1, LS, py.tws[kPlanYF]);
+    fft_passes<NF, 1, false, kThreadsYF, kNB1, kPlanYF, pad_every(NF, kPlanYF, true)>(A, kNB1, LS, py.tws[kPlanYF]);
     // two adjacent Chebyshev rows per thread: one 32-byte store
     for (int idx = threadIdx.x; idx < (kNB1 / 2) * NYA; idx += blockDim.x) {
       const int l0 = 2 * (idx % (kNB1 / 2)), ky = idx / (kNB1 / 2), n = n0 + l0;
@@ -3093,9 +3098,13 @@ void set_smem_named(const char* name, K kernel, size_t bytes) {
 }  // namespace
 
 // ---- launchers ----------------------------------------------------------------
-// Each transform kernel is instantiated for the lengths of the usual grids
-// (compile-time FFT plans); other lengths use the runtime plan.
-#define CORAL_FFT_LENGTHS(X) X(24) X(36) X(48) X(72) X(96) X(144) X(192) X(288) X(384) X(576)
+// Each transform kernel is instantiated for every length 3 N / 2 of a grid (N a
+// multiple of 4, so 2^a 3^b multiples of 6) from 24 to 576; other lengths use the
+// runtime plan, whose radix 2-4 passes ping-pong through shared memory
+// (108 x 64 x 72 modes, run-time against compiled plans, per step: fused z pass 0.43
+// and 0.19 ms, forward x 0.226 and 0.093, inverse x 0.119 and 0.058).
+#define CORAL_FFT_LENGTHS(X) \
+  X(24) X(36) X(48) X(54) X(72) X(96) X(108) X(144) X(162) X(192) X(216) X(288) X(324) X(384) X(432) X(486) X(576)
 
 template <template <int> class L, typename... Args>
 void dispatch_len(int n, Args&&... args) {
@@ -3177,10 +3186,10 @@ template <int NF>
 struct InvZ {
   static void run(const Dims& d, int nf, const double* Y2, double* phys, const FftPlan& pz, const double2* dct_tw,
                   const double* wz, unsigned long long* cfl_bits, cudaStream_t s) {
-    size_t sm = (NF ? 1 : 2) * (kXB3 / 2) * (size_t)d.NZA * sizeof(double2);
+    size_t sm = (NF ? 1 : 2) * (kXB3 / 2) * (size_t)(NF ? line_len(NF, kPlanY, false) : d.NZA) * sizeof(double2);
     set_smem(k_inv_z<NF>, sm);
     dim3 g(nf, (d.NXA + kXB3 - 1) / kXB3, d.NYA);
-    k_inv_z<NF><<<g, kThreads, sm, s>>>(d, Y2, phys, pz, dct_tw, wz, cfl_bits);
+    k_inv_z<NF><<<g, kThreadsIZ, sm, s>>>(d, Y2, phys, pz, dct_tw, wz, cfl_bits);
   }
 };
 template <int NF>

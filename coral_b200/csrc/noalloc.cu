@@ -8,6 +8,7 @@
 // two intermediate arrays of the transform (after the y pass and after the x
 // pass) live in the file-scope __device__ array below, which every GPU that
 // loads this library holds until the process exits.
+#include <algorithm>
 #include <cstring>
 #include <mutex>
 #include <string>
@@ -106,16 +107,31 @@ __device__ __forceinline__ double2 unit_root(double a, int N) {  // exp(-i pi a 
   sincospi(-a / (double)N, &s, &c);
   return make_double2(c, s);
 }
-__global__ void k_twiddles(Tables t) {
-  const int i0 = blockIdx.x * blockDim.x + threadIdx.x, st = gridDim.x * blockDim.x;
-  for (int ax = 0; ax < 3; ++ax) {
-    const int N = t.N[ax];
-    for (int k = i0; k < N; k += st) t.tw[ax][k] = unit_root(2.0 * (double)k, N);
-    for (int pv = 0; pv < 2; ++pv)
-      for (int i = i0; i < t.len[ax][pv]; i += st)
-        t.tws[ax][pv][i] = unit_root(2.0 * (double)pass_tw_index(N, pv, i), N);
+__global__ void k_twiddles(Tables t, int total) {
+  // one entry per thread: the tables' concatenated entries
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
+    int k = i;
+    bool done = false;
+#pragma unroll
+    for (int ax = 0; ax < 3; ++ax) {
+      const int N = t.N[ax];
+      if (!done && k < N) {
+        t.tw[ax][k] = unit_root(2.0 * (double)k, N);
+        done = true;
+      }
+      k -= done ? 0 : N;
+#pragma unroll
+      for (int pv = 0; pv < 2; ++pv) {
+        const int n = t.len[ax][pv];
+        if (!done && k < n) {
+          t.tws[ax][pv][k] = unit_root(2.0 * (double)pass_tw_index(N, pv, k), N);
+          done = true;
+        }
+        k -= done ? 0 : n;
+      }
+    }
+    if (!done) t.dct[k] = unit_root(0.5 * (double)k, t.N[2]);
   }
-  for (int k = i0; k < t.N[2]; k += st) t.dct[k] = unit_root(0.5 * (double)k, t.N[2]);
 }
 
 bool smooth23(int n) {
@@ -191,7 +207,9 @@ extern "C" int coral_spec_to_phys_noalloc(int NX, int NY, int NZ, const double* 
         pl[ax].tws[pv] = tab.tws[ax][pv] = reinterpret_cast<double2*>(base + at);
         at += up256((size_t)tab.len[ax][pv] * sizeof(double2));
       }
-    k_twiddles<<<16, 128, 0, s>>>(tab);
+    int total = tab.N[2];
+    for (int ax = 0; ax < 3; ++ax) total += tab.N[ax] + tab.len[ax][0] + tab.len[ax][1];
+    k_twiddles<<<std::min((total + 63) / 64, 592), 64, 0, s>>>(tab, total);
     const FftPlan &py = pl[0], &px = pl[1], &pz = pl[2];
     launch_inv_y(d, 1, nullptr, StateSet{}, reinterpret_cast<const double2*>(spec), nullptr, nullptr, Y1, py, s);
     launch_inv_x(d, 1, Y1, Y2, px, s);

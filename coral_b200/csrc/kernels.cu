@@ -1632,14 +1632,13 @@ __device__ __forceinline__ bool tpb_block(const FactorArgs& a, int b, TpbBlock& 
   return t.unit < a.nact;
 }
 
-// Assembly of one block of M - dt a(0,0) L into its interleaved band storage:
-// zero fill, then every operator entry added in row order (M before L, slots in
-// order).
+// Rows i0 .. i1 - 1 of one block of M - dt a(0,0) L added to its zeroed interleaved
+// band storage (M before L, slots in order).
 // G: the monomial groups the coefficient registers hold (>= the operators' ngroups)
 template <int G = kMaxGroups>
-__device__ void assemble_tpb(const FactorArgs& a, const TpbBlock& tb) {
+__device__ void assemble_tpb(const FactorArgs& a, const TpbBlock& tb, int i0, int i1) {
   const int cls = tb.cls;
-  const int T = a.Tc, kl = a.kl, ku = a.ku, kv = kl + ku, ldab = a.ldab, RW = a.upw;
+  const int T = a.Tc, kv = a.kl + a.ku, ldab = a.ldab, RW = a.upw;
   const int sid = a.act_list[tb.unit];
   const int kx = sid / a.d.NYA, ky = sid - kx * a.d.NYA;
   double2 cm[G], cl[G];
@@ -1650,9 +1649,7 @@ __device__ void assemble_tpb(const FactorArgs& a, const TpbBlock& tb) {
   }
   double* F = tb.F;
   auto at = [&](int j, int r) -> double& { return F[((size_t)j * ldab + r) * RW]; };
-  for (int j = 0; j < T; ++j)
-    for (int r = 0; r < ldab; ++r) at(j, r) = 0.0;
-  for (int i = 0; i < T; ++i) {
+  for (int i = i0; i < i1; ++i) {
     const int t = a.cls_row[cls * T + i];  // equation row of class position i
     if (t < 0) {
       at(i, kv) = 1.0;  // identity padding
@@ -1679,10 +1676,15 @@ __device__ void assemble_tpb(const FactorArgs& a, const TpbBlock& tb) {
   }
 }
 
+// One thread per block and kAsmRows rows: a row's entries have band places of their
+// own, so the rows are independent (one thread per whole block, zero fill included:
+// 1.88 ms at 96^2 x 48 of the toroidal-poloidal recipe; now 0.34 ms).
+constexpr int kAsmRows = 8;
 template <int G>
 __global__ void __launch_bounds__(kTpbThreads) k_assemble_tpb(FactorArgs a) {
   TpbBlock tb;
-  if (tpb_block(a, blockIdx.x * blockDim.x + threadIdx.x, tb)) assemble_tpb<G>(a, tb);
+  const int i0 = blockIdx.y * kAsmRows;
+  if (tpb_block(a, blockIdx.x * blockDim.x + threadIdx.x, tb)) assemble_tpb<G>(a, tb, i0, min(a.Tc, i0 + kAsmRows));
 }
 
 // DGBTF2 on one block in place in global memory: the algorithm, pivot choice and
@@ -1691,7 +1693,7 @@ __global__ void __launch_bounds__(kTpbThreads) k_assemble_tpb(FactorArgs a) {
 __global__ void __launch_bounds__(kTpbThreads) k_factor_tpb(FactorArgs a) {
   TpbBlock tb;
   if (!tpb_block(a, blockIdx.x * blockDim.x + threadIdx.x, tb)) return;
-  assemble_tpb(a, tb);
+  assemble_tpb(a, tb, 0, a.Tc);
   const int sys = tb.unit, RW = a.upw;
   const int T = a.Tc, kl = a.kl, ku = a.ku, kv = kl + ku, ldab = a.ldab;
   double* F = tb.F;
@@ -1734,105 +1736,136 @@ __global__ void __launch_bounds__(kTpbThreads) k_factor_tpb(FactorArgs a) {
   if (info) atomicMax(a.info + sys, info);
 }
 
-// DGBTF2 on one block (after k_assemble_tpb) with its active band columns in
-// shared memory: the algorithm, pivot choice and update order of k_factor_tpb
-// (the same factors bit for bit), but every factor entry is read from and
-// written to global memory once instead of being updated there up to kl times.
-// At step j the window holds columns j .. j + W - 1 (W = kl + ku + 1: a step
-// touches columns j .. ju, and ju <= j + ku + kl) and column j + W is in
-// flight (cp.async, issued one step ahead into the slot column j - 1 left): a
-// circular buffer of W + 1 slots.  Column j, final after step j, is written
-// back in place.  Each thread's slots are (W + 1) ldab doubles in its own column
-// of shared memory (slot stride blockDim.x <= 32), so the warp's accesses are
-// conflict-free and its global accesses the 256-byte rows of the interleaved
-// layout.  A step's multipliers and each updated column segment are staged in
-// registers (kl <= kFacKl), so that its shared-memory loads issue together.
-constexpr int kFacKl = 16;
-__device__ __forceinline__ void cp_async8(void* smem, const void* gmem) {
-  const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(sa), "l"(gmem) : "memory");
-}
+// DGBTF2 on one block (after k_assemble_tpb) with its active part in shared memory:
+// the algorithm, pivot choice and update order of k_factor_tpb (the same factors bit
+// for bit), but every factor entry is read from and written to global memory once.
+// At step j the active part is rows j .. j+kl by columns j .. j+kv: row j + kl + 1
+// enters when row j, then final, leaves (its columns are exactly the next step's),
+// column j + kv + 1 starts as fill.  Row and column slots are circular, each
+// thread's entries in its own column of shared memory (stride 32: conflict-free).
+// Bound by the latency of a step (one warp issues it), so what counts is how many
+// warps an SM holds: 1.9 KB a thread for the band (9, 23), 3 warps (a window of kv + 2
+// whole band columns took 6.8 KB, 1 warp), and how many loads are ahead of a store:
+// two columns' (2.58 ms at 128^2 x 96 with one column's, now 1.29; 2.39 with the
+// whole-column window).  At 384^2 x 192 the whole factorisation takes 28.9 ms (54.0).
+constexpr int kFacKl = 15, kFacKv = 31;
+template <int KL, int KV>
 __global__ void __launch_bounds__(32) k_factor_win(FactorArgs a) {
   extern __shared__ double fwin[];
-  const int NT = blockDim.x;
+  constexpr int NT = 32;
   TpbBlock tb;
   if (!tpb_block(a, blockIdx.x * NT + threadIdx.x, tb)) return;  // no barriers below
-  const int sys = tb.unit, RW = a.upw;
-  const int T = a.Tc, kl = a.kl, ku = a.ku, kv = kl + ku, ldab = a.ldab, W = kl + ku + 1, W1 = W + 1;
+  const int RW = a.upw, T = a.Tc, kl = a.kl, kv = a.kl + a.ku, ldab = a.ldab, NR = kl + 1, NC = kv + 1;
   double* F = tb.F;
-  double* wz = fwin + threadIdx.x;
-  int j0 = 0, s0 = 0;  // the window's first column and its slot
-  auto slot = [&](int c) { const int q = s0 + (c - j0); return q >= W1 ? q - W1 : q; };
-  auto at = [&](int c, int r) -> double& { return wz[(slot(c) * ldab + r) * NT]; };
-  auto fetch = [&](int c, int sl) {  // column c of the block into slot sl
-    if (c < T) {
-      const double* src = F + (size_t)c * ldab * RW;
-      double* dst = wz + (size_t)sl * ldab * NT;
-      for (int r = 0; r < ldab; ++r) cp_async8(dst + r * NT, src + (size_t)r * RW);
-    }
-  };
-  for (int c = 0; c < W; ++c) fetch(c, c);
-  cp_async_commit();
   unsigned char* P = tb.P;
+  double* w = fwin + threadIdx.x;
+  auto band = [&](int r, int c) -> double& { return F[((size_t)c * ldab + kv + r - c) * RW]; };
+  int r0 = 0, c0 = 0;  // slots of row j and column j
+  auto row = [&](int i) {  // offset of row j + i's slot
+    const int q = r0 + i;
+    return (q >= NR ? q - NR : q) * NC * NT;
+  };
+  auto col = [&](int i) {
+    const int q = c0 + i;
+    return (q >= NC ? q - NC : q) * NT;
+  };
+  for (int r = 0; r <= kl && r < T; ++r)
+    for (int c = 0; c <= kv && c < T; ++c) w[row(r) + col(c)] = band(r, c);
+  const size_t diag = (size_t)(ldab - 1) * RW;  // along a row of the band
+  double* Fj = F + (size_t)kv * RW;              // entry (j, j)
   int ju = 0, info = 0;
   for (int j = 0; j < T; ++j) {
-    j0 = j;
-    fetch(j + W, s0 == 0 ? W1 - 1 : s0 - 1);  // the slot column j - 1 left (the spare at j = 0)
-    cp_async_commit();
-    cp_async_wait<1>();  // columns up to j + W - 1 have landed
-    const int km = min(kl, T - 1 - j);
-    int jp = 0;
-    double mag = fabs(at(j, kv));
-    for (int i = 1; i <= km; ++i) {
-      const double m2 = fabs(at(j, kv + i));
-      if (m2 > mag) { mag = m2; jp = i; }  // first maximum
+    double in[KV + 1];  // row j + kl + 1, columns j + 1 ..
+    {
+      const double* src = Fj + (size_t)ldab * RW + (size_t)kl * RW;
+      const int n = j + kl + 1 < T ? min(kv, T - 2 - j) : -1;
+#pragma unroll
+      for (int q = 0; q <= KV; ++q) in[q] = q <= n ? src[q * diag] : 0.0;
     }
+    const int km = min(kl, T - 1 - j), cj = col(0), rj = row(0);
+    int ro[KL];  // rows j + 1 ..
+#pragma unroll
+    for (int i = 0; i < KL; ++i) ro[i] = i < kl ? row(1 + i) : rj;
+    double m[KL];
+    const double d0 = w[rj + cj];
+    double piv = d0, mag = fabs(d0);
+    int jp = 0, rp = rj;
+#pragma unroll
+    for (int i = 0; i < KL; ++i) m[i] = i < km ? w[ro[i] + cj] : 0.0;
+#pragma unroll
+    for (int i = 0; i < KL; ++i)
+      if (i < km && fabs(m[i]) > mag) {  // first maximum
+        mag = fabs(m[i]);
+        piv = m[i];
+        jp = i + 1;
+        rp = ro[i];
+      }
     P[(size_t)j * RW] = (unsigned char)jp;
-    if (at(j, kv + jp) == 0.0) {
+    double dout = piv;
+    double* dst = Fj;
+    if (piv == 0.0) {
       if (info == 0) info = j + 1;
+      for (int c = 1; c <= kv && j + c < T; ++c) Fj[c * diag] = w[rj + col(c)];
     } else {
-      ju = max(ju, min(j + ku + jp, T - 1));
-      if (jp != 0) {
-        for (int c = j; c <= ju; ++c) {
-          double& p1 = at(c, kv + j + jp - c);
-          double& p0 = at(c, kv + j - c);
-          const double t0 = p0, t1 = p1;
-          p0 = t1;
-          p1 = t0;
+      ju = max(ju, min(j + a.ku + jp, T - 1));
+      const double r = 1.0 / piv;
+      dout = r;
+      // row j + jp comes up, row j goes down; multipliers
+#pragma unroll
+      for (int i = 0; i < KL; ++i)
+        if (i < km) {
+          if (i + 1 == jp) m[i] = d0;
+          m[i] *= r;
         }
-      }
-      const double r = 1.0 / at(j, kv);
-      if (km > 0) {
-        double m[kFacKl];
-        double* cj = wz + ((size_t)s0 * ldab + kv + 1) * NT;
+      // two columns at a time, loads first
+      int cc = col(1);
+#pragma unroll 1
+      for (int c = 1; j + c <= ju; c += 2) {
+        const int c1 = cc, c2 = cc + NT == NC * NT ? 0 : cc + NT;
+        cc = c2 + NT == NC * NT ? 0 : c2 + NT;
+        const bool two = j + c < ju;
+        const double xp1 = w[rp + c1], xj1 = w[rj + c1], xp2 = w[rp + c2], xj2 = w[rj + c2];
+        double v1[KL], v2[KL];
 #pragma unroll
-        for (int i = 0; i < kFacKl; ++i) m[i] = (i < km) ? cj[i * NT] : 0.0;
+        for (int i = 0; i < KL; ++i) {
+          v1[i] = w[ro[i] + c1];
+          v2[i] = w[ro[i] + c2];
+        }
 #pragma unroll
-        for (int i = 0; i < kFacKl; ++i)
+        for (int i = 0; i < KL; ++i)
           if (i < km) {
-            m[i] *= r;
-            cj[i * NT] = m[i];
+            const double x1 = i + 1 == jp ? xj1 : v1[i], x2 = i + 1 == jp ? xj2 : v2[i];
+            w[ro[i] + c1] = x1 - m[i] * xp1;
+            if (two) w[ro[i] + c2] = x2 - m[i] * xp2;
           }
-        for (int c = j + 1; c <= ju; ++c) {
-          double* col = wz + ((size_t)slot(c) * ldab + kv + j - c) * NT;
-          double x[kFacKl + 1];
-#pragma unroll
-          for (int i = 0; i <= kFacKl; ++i) x[i] = (i <= km) ? col[i * NT] : 0.0;
-#pragma unroll
-          for (int i = 0; i < kFacKl; ++i)
-            if (i < km) col[(1 + i) * NT] = x[1 + i] - m[i] * x[0];
-        }
+        dst += diag;
+        *dst = xp1;
+        dst += diag;
+        if (two) *dst = xp2;
       }
-      at(j, kv) = r;
     }
-    // column j is final
-    const double* cw = wz + (size_t)s0 * ldab * NT;
-    double* dst = F + (size_t)j * ldab * RW;
-    for (int q = 0; q < ldab; ++q) dst[(size_t)q * RW] = cw[q * NT];
-    s0 = (s0 + 1 == W1) ? 0 : s0 + 1;
+    *Fj = dout;
+#pragma unroll
+    for (int i = 0; i < KL; ++i)
+      if (i < km) {
+        Fj[(1 + i) * RW] = m[i];
+        w[ro[i] + cj] = 0.0;  // column j + kv + 1: fill
+      }
+    // the next row in row j's slot
+    {
+      int cn = cj;
+#pragma unroll
+      for (int q = 0; q <= KV; ++q)
+        if (q <= kv) {
+          cn = cn + NT == NC * NT ? 0 : cn + NT;
+          w[rj + cn] = in[q];
+        }
+    }
+    Fj += (size_t)ldab * RW;
+    r0 = r0 + 1 == NR ? 0 : r0 + 1;
+    c0 = c0 + 1 == NC ? 0 : c0 + 1;
   }
-  cp_async_wait<0>();
-  if (info) atomicMax(a.info + sys, info);
+  if (info) atomicMax(a.info + tb.unit, info);
 }
 
 // Band rows that are nonzero in any unit, per class and column: one warp per
@@ -2817,14 +2850,20 @@ __global__ void k_zero_step(ZeroArgs a) {
   for (int t = lane; t < T; t += 32) out[t] = b[t];
 }
 
-__global__ void k_zero_factor(ZeroArgs a) {
-  const int s = blockIdx.x;
-  if (s >= a.nsys || threadIdx.x != 0) return;
+// Factorisation of the mean systems (DGBTF2), one warp per system, in shared memory
+// when the bands fit (smem_ok), else in place: lanes own the rows of the assembly
+// and share a column's updates.  (One thread, in place:
+// 0.41 ms at NZ 48; now 0.10 ms.)
+__global__ void __launch_bounds__(32) k_zero_factor(ZeroArgs a, int smem_ok) {
+  extern __shared__ double smd[];
+  const int s = blockIdx.x, lane = threadIdx.x;
+  if (s >= a.nsys) return;
   const ZeroSysDev& z = a.sys[s];
   const int T = z.T, kl = z.kl, ku = z.ku, kv = kl + ku, ldab = z.ldab;
-  double* ab = z.ab;
-  for (size_t e = 0; e < (size_t)T * ldab; ++e) ab[e] = 0.0;
-  for (int t = 0; t < T; ++t) {
+  double* ab = smem_ok ? smd : z.ab;
+  for (int e = lane; e < T * ldab; e += 32) ab[e] = 0.0;
+  __syncwarp();
+  for (int t = lane; t < T; t += 32) {
     for (int k = 0; k < z.M.width; ++k) {
       const double v = z.M.v(t, k);
       if (v == 0.0) continue;
@@ -2838,33 +2877,50 @@ __global__ void k_zero_factor(ZeroArgs a) {
       ab[(size_t)c * ldab + kv + t - c] += a.zsca * v;
     }
   }
+  __syncwarp();
   int ju = 0, info = 0;
   for (int j = 0; j < T; ++j) {
     const int km = min(kl, T - 1 - j);
-    int jp = 0;
+    double* cj = ab + (size_t)j * ldab + kv;
     double best = -1.0;
-    for (int q = 0; q <= km; ++q) {
-      const double v = fabs(ab[(size_t)j * ldab + kv + q]);
+    int jp = 0;
+    for (int q = lane; q <= km; q += 32) {
+      const double v = fabs(cj[q]);
       if (v > best) { best = v; jp = q; }
     }
-    z.dpiv[j] = (unsigned char)jp;
-    if (ab[(size_t)j * ldab + kv + jp] == 0.0) { if (!info) info = j + 1; continue; }
+    for (int o = 16; o > 0; o >>= 1) {  // first maximum
+      const double b2 = __shfl_xor_sync(0xffffffffu, best, o);
+      const int q2 = __shfl_xor_sync(0xffffffffu, jp, o);
+      if (b2 > best || (b2 == best && q2 < jp)) { best = b2; jp = q2; }
+    }
+    if (lane == 0) z.dpiv[j] = (unsigned char)jp;
+    if (cj[jp] == 0.0) { if (!info) info = j + 1; continue; }
     ju = max(ju, min(j + ku + jp, T - 1));
-    if (jp != 0)
-      for (int c = j; c <= ju; ++c) {
+    if (jp != 0) {
+      for (int c = j + lane; c <= ju; c += 32) {
         double* p1 = ab + (size_t)c * ldab + kv + j + jp - c;
         double* p0 = ab + (size_t)c * ldab + kv + j - c;
-        double t0 = *p0; *p0 = *p1; *p1 = t0;
+        const double t0 = *p0;
+        *p0 = *p1;
+        *p1 = t0;
       }
-    const double r = 1.0 / ab[(size_t)j * ldab + kv];
-    for (int q = 1; q <= km; ++q) ab[(size_t)j * ldab + kv + q] *= r;
-    for (int c = j + 1; c <= ju; ++c) {
-      const double rowv = ab[(size_t)c * ldab + kv + j - c];
-      for (int q = 1; q <= km; ++q) ab[(size_t)c * ldab + kv + j + q - c] -= ab[(size_t)j * ldab + kv + q] * rowv;
+      __syncwarp();
     }
-    ab[(size_t)j * ldab + kv] = r;
+    const double r = 1.0 / cj[0];
+    __syncwarp();
+    for (int q = 1 + lane; q <= km; q += 32) cj[q] *= r;
+    __syncwarp();
+    const int nc = ju - j;
+    for (int e = lane; e < nc * km; e += 32) {
+      const int c = j + 1 + e / km, q = 1 + e % km;
+      ab[(size_t)c * ldab + kv + j + q - c] -= cj[q] * ab[(size_t)c * ldab + kv + j - c];
+    }
+    if (lane == 0) cj[0] = r;
+    __syncwarp();
   }
-  a.info[s] = info;
+  if (smem_ok)
+    for (int e = lane; e < T * ldab; e += 32) z.ab[e] = ab[e];
+  if (lane == 0) a.info[s] = info;
 }
 
 // ------------------------------------------------------------------------------
@@ -3611,20 +3667,19 @@ void launch_factor_real(const FactorArgs& a, cudaStream_t s) {
   if (a.nact <= 0) return;
   if (a.tpb) {
     const int nb = a.ncls * a.ngrp * a.upw;
-    // the shared-memory window kernel when a warp's (or at least one thread's)
-    // windows fit in a CTA's shared memory, else the in-place kernel
-    int dev = 0, smax = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&smax, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-    const size_t wbytes = (size_t)(a.kl + a.ku + 2) * a.ldab * sizeof(double);
-    const int nt = (int)std::min<size_t>(32, (size_t)smax / wbytes);
-    if (a.window && a.kl <= kFacKl && nt >= 1) {
-      if (a.M.ngroups <= 8 && a.L.ngroups <= 8)
-        k_assemble_tpb<8><<<(nb + kTpbThreads - 1) / kTpbThreads, kTpbThreads, 0, s>>>(a);
-      else
-        k_assemble_tpb<kMaxGroups><<<(nb + kTpbThreads - 1) / kTpbThreads, kTpbThreads, 0, s>>>(a);
-      set_smem(k_factor_win, (size_t)nt * wbytes);
-      k_factor_win<<<(nb + nt - 1) / nt, nt, (size_t)nt * wbytes, s>>>(a);
+    const size_t sm = (size_t)(a.kl + 1) * (a.kl + a.ku + 1) * 32 * sizeof(double);
+    cudaMemsetAsync(a.abr, 0, (size_t)nb * a.Tc * a.ldab * sizeof(double), s);
+    if (a.window && a.kl <= kFacKl && a.kl + a.ku <= kFacKv) {
+      const dim3 g((nb + kTpbThreads - 1) / kTpbThreads, (a.Tc + kAsmRows - 1) / kAsmRows);
+      if (a.M.ngroups <= 8 && a.L.ngroups <= 8) k_assemble_tpb<8><<<g, kTpbThreads, 0, s>>>(a);
+      else k_assemble_tpb<kMaxGroups><<<g, kTpbThreads, 0, s>>>(a);
+      if (a.kl <= 9 && a.kl + a.ku <= 23) {
+        set_smem(k_factor_win<9, 23>, sm);
+        k_factor_win<9, 23><<<(nb + 31) / 32, 32, sm, s>>>(a);
+      } else {
+        set_smem(k_factor_win<kFacKl, kFacKv>, sm);
+        k_factor_win<kFacKl, kFacKv><<<(nb + 31) / 32, 32, sm, s>>>(a);
+      }
     } else {
       k_factor_tpb<<<(nb + kTpbThreads - 1) / kTpbThreads, kTpbThreads, 0, s>>>(a);
     }
@@ -3646,7 +3701,14 @@ void launch_zero_step(const ZeroArgs& a, cudaStream_t s) {
 }
 void launch_zero_factor(const ZeroArgs& a, cudaStream_t s) {
   if (a.nsys <= 0) return;
-  k_zero_factor<<<a.nsys, 32, 0, s>>>(a);
+  size_t sm = 8;
+  for (int i = 0; i < a.nsys; ++i) sm = std::max(sm, (size_t)a.sys[i].T * a.sys[i].ldab * sizeof(double));
+  int dev = 0, smax = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&smax, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  const bool fits = sm <= (size_t)smax;
+  if (fits) set_smem(k_zero_factor, sm);
+  k_zero_factor<<<a.nsys, 32, fits ? sm : 0, s>>>(a, fits ? 1 : 0);
 }
 void launch_full_dz(const Dims& d, const double2* state, int T, const int* tab_t, const double* tab_v, double dsca,
                     int order, double gap, double2* out, cudaStream_t s) {

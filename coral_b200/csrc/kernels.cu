@@ -2329,27 +2329,46 @@ __device__ __forceinline__ void store_block_rhs(const SolveArgs& a, int sl, int 
   a.work2[((size_t)(c * a.ngrp + (sl >> 5)) * a.Tc + pc) * 32 + (sl & 31)] = v;
 }
 
+// slots k0 .. k0 + 3 of row t.  Slots are filled in order and exact zeros are not
+// stored, so a zero ends the row: a loop over batches that stops after the first
+// batch with one leaves out nothing but further zero terms.
+__device__ __forceinline__ void load_slots(const DevEll& op, int k0, int t, int (&cg)[4], double (&v)[4]) {
+#pragma unroll
+  for (int u = 0; u < 4; ++u) {
+    const bool ok = k0 + u < op.width;
+    cg[u] = ok ? op.cg[(size_t)(k0 + u) * op.rows + t] : 0;
+    v[u] = ok ? op.val[(size_t)(k0 + u) * op.rows + t] : 0.0;
+  }
+}
+
+// S consecutive systems per CTA, so that an operator entry is loaded once for S
+// systems.  Bound by the loads of operator entries and the shared-memory gathers they
+// address (2.5 k instructions a warp, half the cycles without an eligible warp): 143 us
+// at 96^2 x 48 of the toroidal-poloidal recipe with one system, 127 with two.
+template <int S>
 __global__ void __launch_bounds__(kRhsThreads) k_rhs_nl(SolveArgs a, NLArgs n) {
   extern __shared__ double2 shr[];
-  __shared__ double2 cms[kMaxGroups], cns[kMaxGroups];
-  const int sid = blockIdx.x;
-  const int T = a.T, NZ = a.d.NZ;
-  const int kx = sid / a.d.NYA, ky = sid - kx * a.d.NYA;
-  const int aidx = a.act_index[sid];
-  const bool act = aidx >= 0;
-  const bool origin = (kx == 0 && ky == 0);
-  if (threadIdx.x < kMaxGroups) {
-    const int g = threadIdx.x;
-    cms[g] = (g < a.M.ngroups) ? cmul(ipow(a.kx[kx], a.M.gkx[g]), ipow(a.ky[ky], a.M.gky[g])) : zero2();
-    cns[g] = (g < n.NL.ngroups) ? cmul(ipow(a.kx[kx], n.NL.gkx[g]), ipow(a.ky[ky], n.NL.gky[g])) : zero2();
+  __shared__ double2 cms[S][kMaxGroups], cns[S][kMaxGroups];
+  const int T = a.T, NZ = a.d.NZ, nsys = a.d.NXH * a.d.NYA, sid0 = blockIdx.x * S;
+  const int nqz = n.nq * NZ, str = nqz + T;  // per system: [quad][n], then its state
+  bool act[S], any = false;
+#pragma unroll
+  for (int s = 0; s < S; ++s) {
+    act[s] = sid0 + s < nsys && a.act_index[sid0 + s] >= 0;
+    any |= act[s];
   }
-  const size_t base = (size_t)sid * T;
-  const int nqz = act ? n.nq * NZ : 0;
-  double2* qs = shr;         // [quad][n] of this (kx,ky)
-  double2* fs = shr + nqz;   // state of this system
-  {
-    const size_t qstride = (size_t)a.d.NXH * a.d.NYA * NZ;  // between quad vars
-    if (act) {
+  for (int e = threadIdx.x; e < S * kMaxGroups; e += blockDim.x) {
+    const int s = e / kMaxGroups, g = e - s * kMaxGroups, sid = min(sid0 + s, nsys - 1);
+    const int kx = sid / a.d.NYA, ky = sid - kx * a.d.NYA;
+    cms[s][g] = (g < a.M.ngroups) ? cmul(ipow(a.kx[kx], a.M.gkx[g]), ipow(a.ky[ky], a.M.gky[g])) : zero2();
+    cns[s][g] = (g < n.NL.ngroups) ? cmul(ipow(a.kx[kx], n.NL.gkx[g]), ipow(a.ky[ky], n.NL.gky[g])) : zero2();
+  }
+#pragma unroll
+  for (int s = 0; s < S; ++s) {
+    const int sid = sid0 + s;
+    const size_t qstride = (size_t)nsys * NZ;  // between quad vars
+    double2* qs = shr + s * str;
+    if (act[s]) {
       // flat index idx = q NZ + nn, advanced without a division per element
       int q = threadIdx.x / NZ, nn = threadIdx.x - q * NZ;
       for (int idx = threadIdx.x; idx < nqz; idx += blockDim.x) {
@@ -2358,70 +2377,85 @@ __global__ void __launch_bounds__(kRhsThreads) k_rhs_nl(SolveArgs a, NLArgs n) {
         while (nn >= NZ) { nn -= NZ; ++q; }
       }
     }
-    const double2* field = a.field + base;
-    for (int t = threadIdx.x; t < T; t += blockDim.x) fs[t] = field[t];
+    if (sid < nsys) {
+      const double2* field = a.field + (size_t)sid * T;
+      for (int t = threadIdx.x; t < T; t += blockDim.x) qs[nqz + t] = field[t];
+    }
   }
   __syncthreads();
-  const bool zero_out = a.last_stage && !act;
   bool bad = false;
   for (int t = threadIdx.x; t < T; t += blockDim.x) {
-    double2 kh = zero2();
-    if (act) {
+    double2 kh[S], r[S];
+#pragma unroll
+    for (int s = 0; s < S; ++s) kh[s] = r[s] = zero2();
+    if (any) {
       // slots in batches of 4 independent loads; slots are filled in order and
       // exact zeros are not stored, so a zero ends the row
       for (int k0 = 0; k0 < n.NL.width; k0 += 4) {
         int cg[4];
         double v[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          const bool ok = k0 + u < n.NL.width;
-          cg[u] = ok ? n.NL.cg[(size_t)(k0 + u) * n.NL.rows + t] : 0;
-          v[u] = ok ? n.NL.val[(size_t)(k0 + u) * n.NL.rows + t] : 0.0;
-        }
+        load_slots(n.NL, k0, t, cg, v);
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
           if (v[u] != 0.0) {
-            const double2 qh = qs[cg[u] & 0xFFFFFF];  // column = quad * NZ + n
-            kh = cadd(kh, cmul(cns[cg[u] >> 24], make_double2(v[u] * qh.x, v[u] * qh.y)));
+#pragma unroll
+            for (int s = 0; s < S; ++s)
+              if (act[s]) {
+                const double2 qh = shr[s * str + (cg[u] & 0xFFFFFF)];  // column = quad * NZ + n
+                kh[s] = cadd(kh[s], cmul(cns[s][cg[u] >> 24], make_double2(v[u] * qh.x, v[u] * qh.y)));
+              }
           }
         }
         if (v[3] == 0.0) break;
       }
     }
-    // K_hat of the last stage is used only here, from the register (the next step
-    // starts from K_hat_0)
-    if (!a.last_stage) n.Khat[base + t] = kh;
-    double2 r = zero2();
-    if (!origin) {
-#pragma unroll 4
-      for (int k = 0; k < a.M.width; ++k) {
-        const int cg = a.M.cg[(size_t)k * a.M.rows + t];
-        const double v = a.M.val[(size_t)k * a.M.rows + t];
-        const double2 xv = fs[cg & 0xFFFFFF];
-        r = cadd(r, cmul(cms[cg >> 24], make_double2(v * xv.x, v * xv.y)));
+    for (int k0 = 0; k0 < a.M.width; k0 += 4) {
+      int cg[4];
+      double v[4];
+      load_slots(a.M, k0, t, cg, v);
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        if (k0 + u >= a.M.width) break;
+#pragma unroll
+        for (int s = 0; s < S; ++s)
+          if (sid0 + s > 0 && sid0 + s < nsys) {  // not the origin
+            const double2 xv = shr[s * str + nqz + (cg[u] & 0xFFFFFF)];
+            r[s] = cadd(r[s], cmul(cms[s][cg[u] >> 24], make_double2(v[u] * xv.x, v[u] * xv.y)));
+          }
       }
+      if (v[3] == 0.0) break;
     }
 #pragma unroll
-    for (int j = 0; j < kMaxStages - 1; ++j) {  // static indices into the argument arrays
-      if (j < a.nprev) {
-        r = cadd(r, cscale(a.Kstd[j][base + t], a.ca[j]));
-        r = cadd(r, cscale(a.Khat[j][base + t], a.ch[j]));
+    for (int s = 0; s < S; ++s) {
+      const int sid = sid0 + s;
+      if (sid >= nsys) break;
+      const size_t base = (size_t)sid * T;
+      // K_hat of the last stage is used only here, from the register (the next step
+      // starts from K_hat_0)
+      if (!a.last_stage) n.Khat[base + t] = kh[s];
+      double2 b = r[s];
+#pragma unroll
+      for (int j = 0; j < kMaxStages - 1; ++j) {  // static indices into the argument arrays
+        if (j < a.nprev) {
+          b = cadd(b, cscale(a.Kstd[j][base + t], a.ca[j]));
+          b = cadd(b, cscale(a.Khat[j][base + t], a.ch[j]));
+        }
       }
-    }
-    r = cadd(r, cscale(kh, a.ch[a.nprev]));
-    if (act) {
-      if (a.rowflip) r = flip_row(r, a.rowflip[t]);
-      if (a.work2) {  // block layout, class order
-        const int pos = a.row_pos[t], c = pos >= a.Tc ? 1 : 0;
-        store_block_rhs(a, a.slot[sid], c, pos - c * a.Tc, a.row_neg[t], r);
+      b = cadd(b, cscale(kh[s], a.ch[a.nprev]));
+      if (act[s]) {
+        if (a.rowflip) b = flip_row(b, a.rowflip[t]);
+        if (a.work2) {  // block layout, class order
+          const int pos = a.row_pos[t], c = pos >= a.Tc ? 1 : 0;
+          store_block_rhs(a, a.slot[sid], c, pos - c * a.Tc, a.row_neg[t], b);
+        } else {
+          a.work[(size_t)sid * a.wst + (a.row_pos ? a.row_pos[t] : t)] = b;
+        }
       } else {
-        a.work[(size_t)sid * a.wst + (a.row_pos ? a.row_pos[t] : t)] = r;
+        const double2 v = a.last_stage ? zero2() : b;
+        bad |= !(isfinite(v.x) && isfinite(v.y));
+        a.out[base + t] = v;
+        if (a.Kstd_out) a.Kstd_out[base + t] = zero2();
       }
-    } else {
-      const double2 v = zero_out ? zero2() : r;
-      bad |= !(isfinite(v.x) && isfinite(v.y));
-      a.out[base + t] = v;
-      if (a.Kstd_out) a.Kstd_out[base + t] = zero2();
     }
   }
   if (__syncthreads_or(bad) && threadIdx.x == 0) atomicOr(a.flags, 1u);
@@ -2429,48 +2463,63 @@ __global__ void __launch_bounds__(kRhsThreads) k_rhs_nl(SolveArgs a, NLArgs n) {
 
 // ------------------------------------------------------------------------------
 // After the substitutions, one CTA per active system: the solution is staged in
-// shared memory (from the solve's layout), then K_std_i = L x, the stage output
+// shared memory (from the solve's layout), then K_std_i = L x (S systems a CTA, a row
+// ending at its first zero: 82 us -> 71 at 96^2 x 48, toroidal-poloidal), the stage output
 // (the new state in the last stage) and the non-finite check.
 // ------------------------------------------------------------------------------
+template <int S>
 __global__ void __launch_bounds__(kRhsThreads) k_kstd_out(SolveArgs a) {
   extern __shared__ double2 xs[];
-  __shared__ double2 cls[kMaxGroups];
-  const int aidx = blockIdx.x;
-  const int sid = a.act_list[aidx];
-  const int T = a.T;
-  const int kx = sid / a.d.NYA, ky = sid - kx * a.d.NYA;
+  __shared__ double2 cls[S][kMaxGroups];
+  const int a0 = blockIdx.x * S, ns = min(S, a.nact - a0), T = a.T;
   // block solve: the solution is already in out, original order, and
   // only K_std remains (L with its original columns); whole-system solve: the
   // solution is in work (class order = original order), copied to out here
   const bool in_out = a.work2 != nullptr;
   const DevEll& L = in_out ? a.L : a.Lp;
-  if (threadIdx.x < kMaxGroups) {
-    const int g = threadIdx.x;
-    cls[g] = (g < L.ngroups) ? cmul(ipow(a.kx[kx], L.gkx[g]), ipow(a.ky[ky], L.gky[g])) : zero2();
+  for (int e = threadIdx.x; e < ns * kMaxGroups; e += blockDim.x) {
+    const int s = e / kMaxGroups, g = e - s * kMaxGroups, sid = a.act_list[a0 + s];
+    const int kx = sid / a.d.NYA, ky = sid - kx * a.d.NYA;
+    cls[s][g] = (g < L.ngroups) ? cmul(ipow(a.kx[kx], L.gkx[g]), ipow(a.ky[ky], L.gky[g])) : zero2();
   }
-  const size_t base = (size_t)sid * T;
-  {
-    const double2* x = in_out ? a.out + base : a.work + (size_t)sid * a.wst;
-    for (int p = threadIdx.x; p < T; p += blockDim.x) xs[p] = x[p];
+  for (int s = 0; s < ns; ++s) {
+    const int sid = a.act_list[a0 + s];
+    const double2* x = in_out ? a.out + (size_t)sid * T : a.work + (size_t)sid * a.wst;
+    for (int p = threadIdx.x; p < T; p += blockDim.x) xs[s * T + p] = x[p];
   }
   __syncthreads();
   bool bad = false;
   for (int t = threadIdx.x; t < T; t += blockDim.x) {
     if (!in_out) {
-      const double2 v = xs[t];
-      bad |= !(isfinite(v.x) && isfinite(v.y));
-      if (a.out != a.work) a.out[base + t] = v;
+      for (int s = 0; s < ns; ++s) {
+        const double2 v = xs[s * T + t];
+        bad |= !(isfinite(v.x) && isfinite(v.y));
+        if (a.out != a.work) a.out[(size_t)a.act_list[a0 + s] * T + t] = v;
+      }
     }
     if (a.Kstd_out) {
-      double2 ks = zero2();
-#pragma unroll 4
-      for (int k = 0; k < L.width; ++k) {
-        const int cg = L.cg[(size_t)k * L.rows + t];
-        const double lv = L.val[(size_t)k * L.rows + t];
-        const double2 xv = xs[cg & 0xFFFFFF];
-        ks = cadd(ks, cmul(cls[cg >> 24], make_double2(lv * xv.x, lv * xv.y)));
+      double2 ks[S];
+#pragma unroll
+      for (int s = 0; s < S; ++s) ks[s] = zero2();
+      for (int k0 = 0; k0 < L.width; k0 += 4) {
+        int cg[4];
+        double v[4];
+        load_slots(L, k0, t, cg, v);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          if (k0 + u >= L.width) break;
+#pragma unroll
+          for (int s = 0; s < S; ++s)
+            if (s < ns) {
+              const double2 xv = xs[s * T + (cg[u] & 0xFFFFFF)];
+              ks[s] = cadd(ks[s], cmul(cls[s][cg[u] >> 24], make_double2(v[u] * xv.x, v[u] * xv.y)));
+            }
+        }
+        if (v[3] == 0.0) break;
       }
-      a.Kstd_out[base + t] = ks;
+#pragma unroll
+      for (int s = 0; s < S; ++s)
+        if (s < ns) a.Kstd_out[(size_t)a.act_list[a0 + s] * T + t] = ks[s];
     }
   }
   if (__syncthreads_or(bad) && threadIdx.x == 0) atomicOr(a.flags, 1u);
@@ -3009,45 +3058,72 @@ __global__ void k_phys_product(size_t n, const double* a, const double* b, doubl
 // the Chebyshev integration operator trunc(I)[rows 2..NZ, cols 1..NZ-1] (upper
 // triangular: diagonal gap/2 at n = 0, gap/(4(n+1)) beyond; second
 // super-diagonal -gap/(4(n+1)); prepare_chebyshev_integration, :488-505), the
-// last coefficient zero -- into out[kx][ky][n].  One thread per column; the
-// back substitution runs in place with the values it still needs in registers.
+// last coefficient zero -- into out[kx][ky][n].
+// A column's back substitution is two serial chains (n even, n odd: d(n) needs
+// d(n + 2)) of NZ / 2 divides each, so their latency bounds it: a CTA takes cols
+// columns in shared memory, builds and writes them coalesced, and 4 threads a
+// column run the chains (parity, component).  Each chain reads its next c(n + 1)
+// before the step's d(n) overwrite the place.  (One thread a column in global
+// memory: 70 us at 96^2 x 48, now 14.)
 // ------------------------------------------------------------------------------
-__global__ void k_full_dz(Dims d, const double2* state, int T, const int* tab_t, const double* tab_v, double dsca,
-                          int order, double gap, double2* out) {
-  const size_t ncol = (size_t)d.NXH * d.NYA;
-  const int NZ = d.NZ;
-  for (size_t col = (size_t)blockIdx.x * blockDim.x + threadIdx.x; col < ncol; col += (size_t)gridDim.x * blockDim.x) {
-    const double2* sv = state + col * T;
-    double2* o = out + col * NZ;
-    for (int n = 0; n < NZ; ++n) {
-      double2 c = zero2();
-      for (int k = 0; k < kTabW; ++k) {
-        const int tt = tab_t[n * kTabW + k];
-        if (tt >= 0) {
-          const double w = tab_v[n * kTabW + k];
-          const double2 x = sv[tt];
-          c.x += w * x.x;
-          c.y += w * x.y;
-        }
+constexpr int kDzThreads = 128, kDzCols = 8;
+// column stride in shared memory: 4 columns' places in different banks
+__host__ __device__ inline int dz_stride(int NZ) { return NZ + ((2 - NZ) & 7); }
+
+__global__ void __launch_bounds__(kDzThreads) k_full_dz(Dims d, const double2* state, int T, const int* tab_t,
+                                                        const double* tab_v, double dsca, int order, double gap,
+                                                        double2* out, int cols) {
+  extern __shared__ double2 shd[];
+  const int NZ = d.NZ, ld = dz_stride(NZ);
+  double* piv = reinterpret_cast<double*>(shd + (size_t)cols * ld);  // gap / (4 (n + 1))
+  const size_t ncol = (size_t)d.NXH * d.NYA, col0 = (size_t)blockIdx.x * cols;
+  const int nc = (int)(ncol - col0 < (size_t)cols ? ncol - col0 : cols);
+  for (int n = threadIdx.x; n < NZ; n += kDzThreads) piv[n] = gap / (4.0 * (n + 1));
+  for (int e = threadIdx.x; e < nc * NZ; e += kDzThreads) {
+    const int c = e / NZ, n = e - c * NZ;
+    const double2* sv = state + (col0 + c) * T;
+    double2 x = zero2();
+    for (int k = 0; k < kTabW; ++k) {
+      const int tt = tab_t[n * kTabW + k];
+      if (tt >= 0) {
+        const double w = tab_v[n * kTabW + k];
+        const double2 f = sv[tt];
+        x.x += w * f.x;
+        x.y += w * f.y;
       }
-      o[n] = cscale(c, dsca);
     }
+    shd[c * ld + n] = cscale(x, dsca);
+  }
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    const int c = threadIdx.x >> 2, par = (threadIdx.x >> 1) & 1, comp = threadIdx.x & 1;
+    const bool on = c < nc;
+    double* o = reinterpret_cast<double*>(shd + (on ? c : 0) * ld) + comp;
     for (int r = 0; r < order; ++r) {
-      double2 chi = o[NZ - 1];                 // c(n + 1), not yet overwritten
-      double2 dp1 = zero2(), dp2 = zero2();    // d(n + 1), d(n + 2)
-      for (int n = NZ - 2; n >= 0; --n) {
-        const double2 cn = o[n];
-        const double diag = (n == 0) ? 0.5 * gap : gap / (4.0 * (n + 1));
-        const double sup = -gap / (4.0 * (n + 1));
-        const double2 v = (n + 2 <= NZ - 2) ? make_double2(chi.x - sup * dp2.x, chi.y - sup * dp2.y) : chi;
-        const double2 dn = make_double2(v.x / diag, v.y / diag);
-        o[n] = dn;
+      int n = NZ - 2 - par;
+      double chi = n >= 0 ? o[2 * (n + 1)] : 0.0, dp2 = 0.0;  // c(n + 1), d(n + 2)
+      for (int k = 0; k < NZ / 2; ++k, n -= 2) {
+        const double cn = n >= 1 ? o[2 * (n - 1)] : 0.0;
+        __syncwarp();
+        if (n >= 0) {
+          const double diag = (n == 0) ? 0.5 * gap : piv[n];
+          const double sup = -piv[n];
+          const double v = (n + 2 <= NZ - 2) ? chi - sup * dp2 : chi;
+          const double dn = v / diag;
+          if (on) o[2 * n] = dn;
+          dp2 = dn;
+        }
         chi = cn;
-        dp2 = dp1;
-        dp1 = dn;
       }
-      o[NZ - 1] = zero2();
+      __syncwarp();
+      if (on && par == 0) o[2 * (NZ - 1)] = 0.0;
+      __syncwarp();
     }
+  }
+  __syncthreads();
+  for (int e = threadIdx.x; e < nc * NZ; e += kDzThreads) {
+    const int c = e / NZ, n = e - c * NZ;
+    out[(col0 + c) * NZ + n] = shd[c * ld + n];
   }
 }
 
@@ -3580,6 +3656,16 @@ static void group_widths(const DevGEll& G, int w[3]) {
 // threads of a one-CTA-per-system kernel: one per row up to kRhsThreads (a
 // system of 64 rows takes 2 warps, not 8 of which 6 would idle)
 static int rows_threads(int T) { return std::min(kRhsThreads, std::max(32, (T + 31) / 32 * 32)); }
+// Systems a CTA of k_rhs_nl and k_kstd_out: two from 8 an SM on while their rows fit in
+// kPairBytes, below that one (the CTAs no longer fill the chip and a pair only makes
+// each longer).  Toroidal-poloidal recipe, us a step with one | two: 32^2 x 48
+// 302 | 308, 48^2 x 48 404 | 387, 96^2 x 96 1828 | 1793, 128^3 3837 | 3681; four:
+// 96^2 x 48 slower than one.
+constexpr int kPairSys = 8 * 148;
+constexpr size_t kPairBytes = 100 * 1024;
+static bool pair_systems(const SolveArgs& a, size_t bytes_per_system) {
+  return a.d.NXH * a.d.NYA >= kPairSys && 2 * bytes_per_system <= kPairBytes;
+}
 void launch_rhs_nl(const SolveArgs& a, const NLArgs& n, cudaStream_t s) {
   if (a.work2 && a.rhs_win && a.row_pos) {
     if (!a.generic_tiles && a.NLg.valid && a.NLg.ngroups == 3 && a.Mw.width <= 4) {
@@ -3597,8 +3683,13 @@ void launch_rhs_nl(const SolveArgs& a, const NLArgs& n, cudaStream_t s) {
   }
   const int nsys = a.d.NXH * a.d.NYA;
   const size_t sm = ((size_t)n.nq * a.d.NZ + a.T) * sizeof(double2);
-  set_smem(k_rhs_nl, sm);
-  k_rhs_nl<<<nsys, rows_threads(a.T), sm, s>>>(a, n);
+  if (pair_systems(a, sm)) {
+    set_smem(k_rhs_nl<2>, 2 * sm);
+    k_rhs_nl<2><<<(nsys + 1) / 2, rows_threads(a.T), 2 * sm, s>>>(a, n);
+  } else {
+    set_smem(k_rhs_nl<1>, sm);
+    k_rhs_nl<1><<<nsys, rows_threads(a.T), sm, s>>>(a, n);
+  }
 }
 template <int KL, int KV, int UPW>
 static void launch_subst_block(const SolveArgs& a, cudaStream_t s) {
@@ -3655,8 +3746,13 @@ void launch_kstd_out(const SolveArgs& a, cudaStream_t s) {
     return;
   }
   const size_t smx = (size_t)a.T * sizeof(double2);
-  if (smx > 48 * 1024) set_smem(k_kstd_out, smx);
-  k_kstd_out<<<a.nact, rows_threads(a.T), smx, s>>>(a);
+  if (pair_systems(a, smx)) {
+    set_smem(k_kstd_out<2>, 2 * smx);
+    k_kstd_out<2><<<(a.nact + 1) / 2, rows_threads(a.T), 2 * smx, s>>>(a);
+  } else {
+    set_smem(k_kstd_out<1>, smx);
+    k_kstd_out<1><<<a.nact, rows_threads(a.T), smx, s>>>(a);
+  }
 }
 void launch_solve_real(const SolveArgs& a, const NLArgs& n, cudaStream_t s) {
   launch_rhs_nl(a, n, s);
@@ -3712,7 +3808,14 @@ void launch_zero_factor(const ZeroArgs& a, cudaStream_t s) {
 }
 void launch_full_dz(const Dims& d, const double2* state, int T, const int* tab_t, const double* tab_v, double dsca,
                     int order, double gap, double2* out, cudaStream_t s) {
-  k_full_dz<<<grid1d((size_t)d.NXH * d.NYA, 128), 128, 0, s>>>(d, state, T, tab_t, tab_v, dsca, order, gap, out);
+  // columns a CTA: kDzCols, fewer where that many do not fit in 48 KB (any length
+  // whose transforms run fits with one)
+  const size_t colb = dz_stride(d.NZ) * sizeof(double2), tabb = d.NZ * sizeof(double);
+  const int cols = (int)std::max<size_t>(1, std::min<size_t>(kDzCols, (48 * 1024 - std::min<size_t>(tabb, 48 * 1024)) / colb));
+  const size_t sm = cols * colb + tabb, ncol = (size_t)d.NXH * d.NYA;
+  set_smem(k_full_dz, sm);
+  k_full_dz<<<(unsigned)((ncol + cols - 1) / cols), kDzThreads, sm, s>>>(d, state, T, tab_t, tab_v, dsca, order, gap, out,
+                                                                         cols);
 }
 void launch_zero_dz(int NZ, const double* state, const int* tab_t, const double* tab_v, double dsca, int order,
                     double gap, double* out, cudaStream_t s) {

@@ -100,6 +100,7 @@ struct KSys {
   unsigned char *row_neg = nullptr, *col_neg = nullptr;
   unsigned long long* cmask = nullptr;
   double *lpack = nullptr, *upack = nullptr;
+  int fac_chunk = 1;  // groups of each class in abr (block layout)
   uint4* finfo = nullptr;
   uint4* binfo = nullptr;
   int* ptot = nullptr;
@@ -854,7 +855,17 @@ void setup(coral_handle* h, const std::string& eqs, const std::string& pars, con
       k.row_neg = mem.upload(k.ops.row_neg);
       k.col_neg = mem.upload(k.ops.col_neg);
       const size_t ng = 2 * (size_t)k.ngrp, cols = ng * k.Tc, kv = (size_t)k.kl_s + k.ku_s;
-      k.abr = mem.get<double>(cols * k.ldab_s * k.upw);
+      // the factorisation's workspace: all groups, or a 16th of them where that would
+      // take more than a quarter of the memory left (the packed factors, as large,
+      // and the transforms' buffers are still to come)
+      const size_t per_group = 2 * (size_t)k.Tc * k.ldab_s * k.upw;
+      size_t mfree = 0, mtotal = 0;
+      CK(cudaMemGetInfo(&mfree, &mtotal));
+      k.fac_chunk = std::max(k.ngrp, 1);
+      if (per_group * k.ngrp * sizeof(double) > mfree / 4) k.fac_chunk = (k.ngrp + 15) / 16;
+      if (const char* e = std::getenv("CORAL_FACTOR_CHUNK"); e && std::atoi(e) > 0)
+        k.fac_chunk = std::min(k.fac_chunk, std::atoi(e));
+      k.abr = mem.get<double>(per_group * k.fac_chunk);
       k.lpack = mem.get<double>(cols * std::max(k.kl_s, 1) * k.upw);
       k.upack = mem.get<double>(cols * (kv + 1) * k.upw);
       k.dpiv = mem.get<unsigned char>(cols * k.upw);
@@ -866,10 +877,6 @@ void setup(coral_handle* h, const std::string& eqs, const std::string& pars, con
       // padding lanes have factors of their own (zeros) and zero right-hand sides
       CK(cudaMemset(k.work2, 0, cols * 32 * sizeof(double2)));
       CK(cudaMemset(k.dpiv, 0, cols * k.upw));
-      for (int c = 0; c < 2; ++c) {
-        const size_t last = (size_t)c * k.ngrp + k.ngrp - 1, n = (size_t)k.Tc * k.ldab_s * k.upw;
-        if (k.ngrp > 0) CK(cudaMemset(k.abr + last * n, 0, n * sizeof(double)));
-      }
     } else {
       if (k.real) k.abr = mem.get<double>((size_t)h->nact * k.Tc * k.ldab_s);
       else k.ab = mem.get<double2>((size_t)h->nact * k.T * k.ldab);
@@ -1535,6 +1542,8 @@ void factorize(coral_handle* h, double dt) {
     fa.window = h->tune.factor_window;
     fa.upw = k.upw;
     fa.ngrp = k.ngrp;
+    fa.g0 = 0;
+    fa.gn = k.fac_chunk;
     fa.cmask = k.cmask;
     fa.lpack = k.lpack;
     fa.upack = k.upack;

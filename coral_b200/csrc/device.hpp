@@ -316,6 +316,9 @@ struct FactorArgs {
   // nact their number): factors abr[((G Tc + j) ldab + r) upw + unit], packed for
   // the substitution into lpack / upack by k_pack
   int tpb, upw, ngrp;
+  // abr holds the groups g0 .. g0 + gn - 1 of each class (all, or a chunk of them:
+  // see launch_factor_real)
+  int g0, gn;
   int window;            // block layout: 1 shared-memory band window, 0 in place in global memory
   unsigned long long* cmask;  // [2 Tc] per class and column, the band rows nonzero in any unit
   double* lpack;

@@ -1624,11 +1624,12 @@ struct TpbBlock {
 };
 __device__ __forceinline__ bool tpb_block(const FactorArgs& a, int b, TpbBlock& t) {
   const int G = b / a.upw, lane = b - G * a.upw;
-  if (G >= a.ncls * a.ngrp) return false;
-  t.cls = G / a.ngrp;
-  t.unit = (G - t.cls * a.ngrp) * a.upw + lane;
+  if (G >= a.ncls * a.gn) return false;
+  t.cls = G / a.gn;
+  const int g = a.g0 + G - t.cls * a.gn;
+  t.unit = g * a.upw + lane;
   t.F = a.abr + (size_t)G * a.Tc * a.ldab * a.upw + lane;
-  t.P = a.dpiv + (size_t)G * a.Tc * a.upw + lane;
+  t.P = a.dpiv + ((size_t)t.cls * a.ngrp + g) * a.Tc * a.upw + lane;
   return t.unit < a.nact;
 }
 
@@ -1876,7 +1877,7 @@ __global__ void __launch_bounds__(256) k_mask_cols(FactorArgs a) {
   const int G = blockIdx.x, j = blockIdx.y * 8 + w;
   const int T = a.Tc, ldab = a.ldab;
   if (j >= T) return;
-  const int cls = G / a.ngrp, u0 = (G - cls * a.ngrp) * a.upw;
+  const int cls = G / a.gn, u0 = (a.g0 + G - cls * a.gn) * a.upw;
   const bool ok = lane < a.upw && u0 + lane < a.nact;
   const double* F = a.abr + ((size_t)G * T + j) * ldab * a.upw + (ok ? lane : 0);
   unsigned long long bits = 0;
@@ -1948,7 +1949,7 @@ __global__ void __launch_bounds__(256) k_pack(FactorArgs a) {
   const int G = blockIdx.x, k = blockIdx.y * 8 + w;
   const int T = a.Tc, kv = a.kl + a.ku, ldab = a.ldab, RW = a.upw;
   if (k >= T) return;
-  const int cls = G / a.ngrp, g = G - cls * a.ngrp;
+  const int cls = G / a.gn, g = a.g0 + G - cls * a.gn;
   const double* F = a.abr + (size_t)G * T * ldab * RW;
   const int half = lane / RW, ln = lane - half * RW, per = 32 / RW;  // rows a warp copies at a time
   {
@@ -3759,31 +3760,47 @@ void launch_solve_real(const SolveArgs& a, const NLArgs& n, cudaStream_t s) {
   launch_subst(a, s);
   launch_kstd_out(a, s);
 }
-void launch_factor_real(const FactorArgs& a, cudaStream_t s) {
+// the band factorisation of the groups that a.abr holds
+static void launch_factor_blocks(const FactorArgs& a, cudaStream_t s) {
+  const int nb = a.ncls * a.gn * a.upw;
+  const size_t sm = (size_t)(a.kl + 1) * (a.kl + a.ku + 1) * 32 * sizeof(double);
+  cudaMemsetAsync(a.abr, 0, (size_t)nb * a.Tc * a.ldab * sizeof(double), s);
+  if (a.window && a.kl <= kFacKl && a.kl + a.ku <= kFacKv) {
+    const dim3 g((nb + kTpbThreads - 1) / kTpbThreads, (a.Tc + kAsmRows - 1) / kAsmRows);
+    if (a.M.ngroups <= 8 && a.L.ngroups <= 8) k_assemble_tpb<8><<<g, kTpbThreads, 0, s>>>(a);
+    else k_assemble_tpb<kMaxGroups><<<g, kTpbThreads, 0, s>>>(a);
+    if (a.kl <= 9 && a.kl + a.ku <= 23) {
+      set_smem(k_factor_win<9, 23>, sm);
+      k_factor_win<9, 23><<<(nb + 31) / 32, 32, sm, s>>>(a);
+    } else {
+      set_smem(k_factor_win<kFacKl, kFacKv>, sm);
+      k_factor_win<kFacKl, kFacKv><<<(nb + 31) / 32, 32, sm, s>>>(a);
+    }
+  } else {
+    k_factor_tpb<<<(nb + kTpbThreads - 1) / kTpbThreads, kTpbThreads, 0, s>>>(a);
+  }
+}
+// Block layout: the union masks need every group's factors before any is packed.
+// With a workspace of all groups (chunk = ngrp) each group is factored once; with a
+// smaller one, where memory is short, twice: for the masks, then for the packing.
+void launch_factor_real(const FactorArgs& full, cudaStream_t s) {
+  FactorArgs a = full;
   if (a.nact <= 0) return;
   if (a.tpb) {
-    const int nb = a.ncls * a.ngrp * a.upw;
-    const size_t sm = (size_t)(a.kl + 1) * (a.kl + a.ku + 1) * 32 * sizeof(double);
-    cudaMemsetAsync(a.abr, 0, (size_t)nb * a.Tc * a.ldab * sizeof(double), s);
-    if (a.window && a.kl <= kFacKl && a.kl + a.ku <= kFacKv) {
-      const dim3 g((nb + kTpbThreads - 1) / kTpbThreads, (a.Tc + kAsmRows - 1) / kAsmRows);
-      if (a.M.ngroups <= 8 && a.L.ngroups <= 8) k_assemble_tpb<8><<<g, kTpbThreads, 0, s>>>(a);
-      else k_assemble_tpb<kMaxGroups><<<g, kTpbThreads, 0, s>>>(a);
-      if (a.kl <= 9 && a.kl + a.ku <= 23) {
-        set_smem(k_factor_win<9, 23>, sm);
-        k_factor_win<9, 23><<<(nb + 31) / 32, 32, sm, s>>>(a);
-      } else {
-        set_smem(k_factor_win<kFacKl, kFacKv>, sm);
-        k_factor_win<kFacKl, kFacKv><<<(nb + 31) / 32, 32, sm, s>>>(a);
-      }
-    } else {
-      k_factor_tpb<<<(nb + kTpbThreads - 1) / kTpbThreads, kTpbThreads, 0, s>>>(a);
-    }
-    const int ng = a.ncls * a.ngrp;
+    const int chunk = full.gn;
+    const auto rows = [&](int gn) { return dim3(full.ncls * gn, (full.Tc + 7) / 8); };
     cudaMemsetAsync(a.cmask, 0, (size_t)a.ncls * a.Tc * sizeof(unsigned long long), s);
-    k_mask_cols<<<dim3(ng, (a.Tc + 7) / 8), 256, 0, s>>>(a);
+    for (a.g0 = 0; a.g0 < a.ngrp; a.g0 += chunk) {
+      a.gn = std::min(chunk, a.ngrp - a.g0);
+      launch_factor_blocks(a, s);
+      k_mask_cols<<<rows(a.gn), 256, 0, s>>>(a);
+    }
     k_pack_info<<<a.ncls, 32, 0, s>>>(a);
-    k_pack<<<dim3(ng, (a.Tc + 7) / 8), 256, 0, s>>>(a);
+    for (a.g0 = 0; a.g0 < a.ngrp; a.g0 += chunk) {
+      a.gn = std::min(chunk, a.ngrp - a.g0);
+      if (chunk < a.ngrp) launch_factor_blocks(a, s);
+      k_pack<<<rows(a.gn), 256, 0, s>>>(a);
+    }
     return;
   }
   k_factor_real<<<dim3((a.nact + kWPB - 1) / kWPB, a.ncls), kWPB * 32, 0, s>>>(a);

@@ -35,3 +35,14 @@ def test_window_and_in_place_factors_agree(name, grid):
     eq, par = _recipe(name), params(*grid, dt=1e-5)
     for a, b in zip(_run(eq, par, False), _run(eq, par, True)):
         assert np.isfinite(a).all() and np.array_equal(a, b)
+
+
+# a workspace of 1 or 3 groups at a time: chunks of one, a last one that is partial
+@pytest.mark.parametrize("chunk", [1, 3])
+@pytest.mark.parametrize("name", ["rbc_noslip_ra1e5", "rrbc_stressfree_ek1e-4_ra5e7"])
+def test_chunked_factorisation_agrees(name, chunk, monkeypatch):
+    eq, par = _recipe(name), params(24, 24, 16, dt=1e-5)
+    whole = _run(eq, par, False)
+    monkeypatch.setenv("CORAL_FACTOR_CHUNK", str(chunk))
+    for a, b in zip(whole, _run(eq, par, False)):
+        assert np.array_equal(a, b)

@@ -2944,8 +2944,10 @@ __global__ void __launch_bounds__(32) k_zero_factor(ZeroArgs a, int smem_ok) {
       if (b2 > best || (b2 == best && q2 < jp)) { best = b2; jp = q2; }
     }
     if (lane == 0) z.dpiv[j] = (unsigned char)jp;
-    if (cj[jp] == 0.0) { if (!info) info = j + 1; continue; }
+    // (from the register all lanes share: lane 0 overwrites cj[jp] below)
+    if (best == 0.0) { if (!info) info = j + 1; continue; }
     ju = max(ju, min(j + ku + jp, T - 1));
+    __syncwarp();  // every lane has read the column
     if (jp != 0) {
       for (int c = j + lane; c <= ju; c += 32) {
         double* p1 = ab + (size_t)c * ldab + kv + j + jp - c;

@@ -3229,6 +3229,22 @@ void set_smem_named(const char* name, K kernel, size_t bytes) {
 }
 // (variadic so that template argument lists pass through; the text names the call)
 #define set_smem(...) set_smem_named(#__VA_ARGS__, __VA_ARGS__)
+// CTAs with that much dynamic shared memory that an SM's shared memory holds (0: refused)
+template <typename K>
+int resident_by_smem(K kernel, size_t bytes) {
+  cudaFuncAttributes fa;
+  if (cudaFuncGetAttributes(&fa, kernel) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  int dev = 0, optin = 0, sm = 0, reserved = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  cudaDeviceGetAttribute(&sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev);
+  cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, dev);
+  const size_t total = fa.sharedSizeBytes + bytes;
+  return total > (size_t)optin ? 0 : (int)((size_t)sm / (total + reserved));
+}
 
 }  // namespace
 
@@ -3340,11 +3356,20 @@ struct FwdZ {
 template <int NF>
 struct ZFused {
   template <int FB>
+  static size_t bytes(int nf, const Dims& d) {
+    const size_t lines = (size_t)nf * kZPairs + FB + (NF ? 0 : std::max(kZLines, FB));
+    return lines * (NF ? line_len(NF, kPlanHot, false) : d.NZA) * sizeof(double2);
+  }
+  // CTAs that an SM's shared memory holds
+  template <int FB>
+  static int resident(int nf, const Dims& d) {
+    return resident_by_smem(k_z_fused<NF, FB>, bytes<FB>(nf, d));
+  }
+  template <int FB>
   static void go(const Dims& d, int nf, const QuadDesc& q, const double* Y2, double* Q2, const FftPlan& pz,
                  const double2* dct_tw, const double* wz, const double* wzinv, unsigned long long* cfl_bits,
                  double* ke_partial, int y0, int ny, cudaStream_t s) {
-    const size_t lines = (size_t)nf * kZPairs + FB + (NF ? 0 : std::max(kZLines, FB));
-    const size_t sm = lines * (NF ? line_len(NF, kPlanHot, false) : d.NZA) * sizeof(double2);
+    const size_t sm = bytes<FB>(nf, d);
     set_smem(k_z_fused<NF, FB>, sm);
     dim3 g((d.NXA + 2 * kZPairs - 1) / (2 * kZPairs), ny);
     k_z_fused<NF, FB><<<g, z_threads_fused(NF, FB), sm, s>>>(d, nf, q, Y2, Q2, pz, dct_tw, wz, wzinv, cfl_bits,
@@ -3357,8 +3382,15 @@ struct ZFused {
       ZFused<0>::run(d, nf, q, Y2, Q2, pz, dct_tw, wz, wzinv, cfl_bits, ke_partial, batch6, y0, ny, s);
       return;
     }
-    if (batch6 && nf <= 4) go<6>(d, nf, q, Y2, Q2, pz, dct_tw, wz, wzinv, cfl_bits, ke_partial, y0, ny, s);
-    else go<kZFwd>(d, nf, q, Y2, Q2, pz, dct_tw, wz, wzinv, cfl_bits, ke_partial, y0, ny, s);
+    // Up to 4 full variables batches of 6 lines (unless the variant asks for 9); above
+    // that of 9, but of 6 where an SM's shared memory then holds two CTAs and not one (ms
+    // a step with 9 | 6 lines: 7 variables at 96^2 x 192 9.06 | 8.57, 5 at 64^2 x 256
+    // 2.88 | 2.70), or one and not none (7 or 8 variables at NZ 384).
+    const bool six = batch6 && (nf <= 4 || (resident<kZFwd>(nf, d) < 2 && resident<6>(nf, d) > resident<kZFwd>(nf, d)));
+    if (six || resident<kZFwd>(nf, d) < 1)
+      go<6>(d, nf, q, Y2, Q2, pz, dct_tw, wz, wzinv, cfl_bits, ke_partial, y0, ny, s);
+    else
+      go<kZFwd>(d, nf, q, Y2, Q2, pz, dct_tw, wz, wzinv, cfl_bits, ke_partial, y0, ny, s);
   }
 };
 template <int NF>

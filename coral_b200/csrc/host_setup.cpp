@@ -635,6 +635,7 @@ SystemOps assemble_system(const Geometry& g, const Recipe& r, const CoupledSet& 
     return it->second;
   };
 
+  std::vector<int> nonzero;  // entries of a row of the integration operator, in order
   auto build = [&](const std::vector<Piece>& pieces, EllOp& op) {
     std::vector<Triplet> tr;
     for (const Piece& p : pieces) {
@@ -645,10 +646,13 @@ SystemOps assemble_system(const Geometry& g, const Recipe& r, const CoupledSet& 
       int nc = int(Sv[0].size());
       for (int rr = 0; rr < o.eq_size[p.iEqn]; ++rr) {
         const auto& crow = C[o_e + rr];
+        nonzero.clear();
+        for (int n = 0; n < NZ; ++n)
+          if (crow[n] != 0.0) nonzero.push_back(n);
         for (int c = 0; c < nc; ++c) {
           double acc = 0.0;
-          for (int n = 0; n < NZ; ++n)
-            if (crow[n] != 0.0 && Sv[n][c] != 0.0) acc += crow[n] * Sv[n][c];
+          for (int n : nonzero)
+            if (Sv[n][c] != 0.0) acc += crow[n] * Sv[n][c];
           if (acc != 0.0) tr.push_back({o.eq_pos[p.iEqn][rr], o.var_pos[p.jVar][c], grp, p.dsca * acc});
         }
       }

@@ -162,8 +162,25 @@ __host__ __device__ constexpr PlanR make_planr2(int N) {
   if (N == 576) return PlanR{2, {24, 24}};
   return make_planr(N);
 }
-// plan variant PV: 0 = make_planr, 1 = make_planr2
-__host__ __device__ constexpr PlanR plan_of(int N, int PV) { return PV ? make_planr2(N) : make_planr(N); }
+// make_planr's radices in passes of at most 12 elements: the forward z pass keeps 64
+// registers a thread, with which 27-element butterflies spill 1 to 2.4 KB (one | nine
+// variables of a 144 x 144 grid, us, run-time plan, 27-element passes, these: 162
+// points 50 | 193, 41 | 181, 38 | 160; 216: 53 | 238, 48 | 242, 48 | 215; 324: 63 |
+// 378, 100 | 481, 64 | 318; 432: 73 | 600, 115 | 704, 92 | 516)
+__host__ __device__ constexpr PlanR make_planr3(int N) {
+  switch (N) {
+    case 162: return PlanR{3, {303, 303, 2}};
+    case 216: return PlanR{3, {403, 3, 302}};
+    case 324: return PlanR{3, {4, 303, 303}};
+    case 432: return PlanR{3, {4, 403, 303}};
+    default: return make_planr(N);
+  }
+}
+// plan variant PV: 0 = make_planr, 1 = make_planr2, 2 = make_planr3 (its radices are
+// make_planr's in the same order, so the twiddle tables of variant 0 serve it)
+__host__ __device__ constexpr PlanR plan_of(int N, int PV) {
+  return PV == 0 ? make_planr(N) : PV == 1 ? make_planr2(N) : make_planr3(N);
+}
 
 // cos / sin of 2 pi m / 16 and 2 pi m / 9, from the mathematics (40-digit values)
 #define CORAL_C16_1 0.923879532511286756128183189396788287   // cos(pi/8)
@@ -587,13 +604,13 @@ __device__ __forceinline__ double2* fft_lines_ld(double2* A, double2* B, int nl,
 }
 
 // The same of lines already in A (unpadded; the caller has synchronised)
-template <int NC, bool INV, int NT, int NLMAX>
+template <int NC, bool INV, int NT, int NLMAX, int PV = 0>
 __device__ __forceinline__ double2* fft_lines_n(double2* A, double2* B, int nl, int LS, const FftPlan& p) {
   if constexpr (NC == 0) {
     return fft_lines<INV>(A, B, nl, LS, p);
   } else {
-    static_assert(make_planr(NC).nst > 0, "transform length must be 2^a 3^b");
-    fft_passes<NC, 0, INV, NT, NLMAX>(A, nl, LS, p.tws[0]);
+    static_assert(plan_of(NC, PV).nst > 0, "transform length must be 2^a 3^b");
+    fft_passes<NC, 0, INV, NT, NLMAX, PV>(A, nl, LS, p.tws[PV % 2]);
     return A;
   }
 }

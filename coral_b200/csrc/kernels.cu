@@ -38,6 +38,7 @@ constexpr int kThreads = 256;
 // chains (measured at 384^2 x 192)
 constexpr int kPlanHot = 1;
 constexpr int kPlanY = 0;
+constexpr int kPlanFZ = 2;  // separate forward z pass
 // x / y passes: threads per CTA for nl lines of a compiled length N, the most
 // that any pass keeps busy, rounded up to whole warps: one butterfly per thread,
 // of radix 2, 3 and 4 as many as make 8 or 9 elements (one radix-3 butterfly each
@@ -533,7 +534,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocksZ) k_fwd_z(Dims d, int nf,
       A[qi * N + m] = make_double2(pa, pb);
     }
     __syncthreads();
-    const double2* R = fft_lines_n<NF, false, kThreads, kQC>(A, B, nc, N, pz);
+    const double2* R = fft_lines_n<NF, false, kThreads, kQC, kPlanFZ>(A, B, nc, N, pz);
     for (int idx = threadIdx.x; idx < nc * d.NZ; idx += blockDim.x) {
       const int qi = idx / d.NZ, n = idx - qi * d.NZ;
       const double2 Z = R[qi * N + n];
@@ -3347,6 +3348,11 @@ template <int NF>
 struct FwdZ {
   static void run(const Dims& d, int nf, const QuadDesc& q, const double* phys, double* Q2, const FftPlan& pz,
                   const double2* dct_tw, const double* wz, double* ke_partial, cudaStream_t s) {
+    // one variable of 432 points: few of the threads have a butterfly, and the run-time
+    // plan's smaller ones are faster (73 us, compiled 92 us)
+    if constexpr (NF == 432) {
+      if (q.nq == 1) return FwdZ<0>::run(d, nf, q, phys, Q2, pz, dct_tw, wz, ke_partial, s);
+    }
     size_t sm = (size_t)nf * d.NZA * sizeof(double2) + (NF ? 1 : 2) * (size_t)std::min(q.nq, kQC) * d.NZA * sizeof(double2);
     set_smem(k_fwd_z<NF>, sm);
     dim3 g((d.NXA + 1) / 2, d.NYA);

@@ -52,12 +52,14 @@ struct NetDev {
 // The network's products on the tensor cores, in FP32 precision: weights are
 // BF16 as they are; an FP32 activation (or gradient) is the exact sum of three
 // BF16 numbers, h = bf16(h) + bf16(rest) + bf16(rest), so h W is three BF16
-// products with FP32 accumulation.  (Relative error of tau against FP64 1.5e-7;
-// of scalar FP32 sums in one chain 2.8e-7.)
+// products with FP32 accumulation.  (Relative error of tau against FP64, rms, for
+// inputs of 1 | 0.1 | 0.01 | 1e-5: 1.5e-7 | 1.8e-7 | 1.9e-7 | 1.9e-7; of scalar FP32
+// sums in one chain 2.8e-7 | 3.3e-7 | 3.1e-7 | 3.1e-7.)
 //
-// A warp takes 16 points through all layers with its activations in registers: the accumulator layout of mma.m16n8k16 (rows = points, columns =
-// features) is the A-operand layout of the next layer's k step.  Lane = 4 g + q
-// holds rows g and g + 8 and columns 2 q, 2 q + 1 of every 8-column tile.
+// A warp takes 16 points through all layers with its activations in registers: the
+// accumulator layout of mma.m16n8k16 (rows = points, columns = features) is the
+// A-operand layout of the next layer's k step.  Lane = 4 g + q holds rows g and g + 8
+// and columns 2 q, 2 q + 1 of every 8-column tile.
 // Legacy MMAs, not tcgen05: their accumulators stay in registers from layer to
 // layer, and the tensor pipe is a third busy; the issue slots (48%: splitting,
 // tanh, the stencil's addresses) and the instruction cache bound the kernel.  One
@@ -82,6 +84,20 @@ __device__ __forceinline__ void mma16816(float (&d)[4], const unsigned (&a)[4], 
       : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b.x), "r"(b.y), "f"(c[0]), "f"(c[1]), "f"(c[2]), "f"(c[3]));
 }
+// two floats as one operand of the packed FP32 instructions
+__device__ __forceinline__ unsigned long long pair2(float a, float b) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ void unpair2(unsigned long long p, float& a, float& b) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(p));
+}
+__device__ __forceinline__ unsigned long long add2(unsigned long long a, unsigned long long b) {
+  unsigned long long r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
 // c += a b, a in three planes: the step's products are summed from zero, smallest
 // plane first, and added to c in one rounding (the tensor core's own additions
 // truncate: with c as their accumulator the error against FP64 doubled)
@@ -92,7 +108,7 @@ __device__ __forceinline__ void mma_planes(float (&c)[4], const unsigned (&a)[3]
   mma16816(t1, a[1], b, t2);
   mma16816(t0, a[0], b, t1);
 #pragma unroll
-  for (int e = 0; e < 4; ++e) c[e] += t0[e];
+  for (int e = 0; e < 4; e += 2) unpair2(add2(pair2(c[e], c[e + 1]), pair2(t0[e], t0[e + 1])), c[e], c[e + 1]);
 }
 __device__ __forceinline__ unsigned pack2(float lo, float hi) {
   unsigned r;
@@ -242,12 +258,51 @@ __device__ __forceinline__ void hidden_product(float (&c)[NT][4], const float (&
   }
 }
 
-// tanh x = (e^{2x} - 1) / (e^{2x} + 1), absolute error about 1e-7 (the argument cut
-// where the quotient rounds to 1; NaN stays): a third of tanhf's instructions, the
-// largest part of the kernel's
-__device__ __forceinline__ float tanh_exp(float x) {
-  const float t = exp2f(2.8853900817779268f * (x > 15.0f ? 15.0f : x));  // 2 / ln 2
-  return __fdividef(t - 1.0f, t + 1.0f);
+// tanh of two values at once: an odd polynomial below 0.5 (least-maximum fit of the
+// relative error to tanh, 1.5e-8, by iteratively reweighted least squares), above it
+// 1 - 2 / (e^{2|x|} + 1), where the subtraction loses nothing, so relative accuracy
+// holds down to the smallest x.  Cut at 15, where the quotient is below half a last
+// bit; NaN stays.  Packed in pairs, as the issue slots bound the kernel (96 x 96 x 72
+// points: tanhf 443 us, this 390 with the sums of mma_planes in pairs too, 410 without).
+__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
+  unsigned long long r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ unsigned long long mul2(unsigned long long a, unsigned long long b) {
+  unsigned long long r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ float min_nan(float a, float b) {
+  float r;
+  asm("min.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ float ex2_approx(float a) {
+  float r;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(a));
+  return r;
+}
+__device__ __forceinline__ float rcp_approx(float a) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(a));
+  return r;
+}
+__device__ __forceinline__ void tanh_pair(float& x0, float& x1) {
+  const float a0 = fabsf(x0), a1 = fabsf(x1);
+  const unsigned long long x = pair2(x0, x1), y = mul2(x, x);
+  unsigned long long p = fma2(pair2(0.017241491f, 0.017241491f), y, pair2(-0.053045493f, -0.053045493f));
+  p = fma2(p, y, pair2(0.13325879f, 0.13325879f));
+  p = fma2(p, y, pair2(-0.33333144f, -0.33333144f));
+  float s0, s1, t0, t1, q0, q1;
+  unpair2(fma2(x, mul2(p, y), x), s0, s1);
+  constexpr float k = 2.8853900817779268f;  // 2 / ln 2
+  unpair2(mul2(pair2(min_nan(a0, 15.0f), min_nan(a1, 15.0f)), pair2(k, k)), t0, t1);
+  unpair2(add2(pair2(ex2_approx(t0), ex2_approx(t1)), pair2(1.0f, 1.0f)), t0, t1);
+  unpair2(fma2(pair2(rcp_approx(t0), rcp_approx(t1)), pair2(-2.0f, -2.0f), pair2(1.0f, 1.0f)), q0, q1);
+  x0 = a0 < 0.5f ? s0 : copysignf(q0, x0);
+  x1 = a1 < 0.5f ? s1 : copysignf(q1, x1);
 }
 
 // Inference on a grid: point p is grid point p (linear [y][x][z]) of fields
@@ -290,7 +345,7 @@ __global__ void __launch_bounds__(kInferThreads, kInferCtas) k_closure_infer(Net
 #pragma unroll
       for (int n = 0; n < 8; ++n)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) h[n][e] = tanh_exp(h[n][e]);
+        for (int e = 0; e < 4; e += 2) tanh_pair(h[n][e], h[n][e + 1]);
       hidden_product<8>(c, h, Bs + (layer ? fW2 : fW1) * 32, lane);
 #pragma unroll
       for (int n = 0; n < 8; ++n)
@@ -300,7 +355,7 @@ __global__ void __launch_bounds__(kInferThreads, kInferCtas) k_closure_infer(Net
 #pragma unroll
     for (int n = 0; n < 8; ++n)
 #pragma unroll
-      for (int e = 0; e < 4; ++e) h[n][e] = tanh_exp(h[n][e]);
+      for (int e = 0; e < 4; e += 2) tanh_pair(h[n][e], h[n][e + 1]);
     float y[2][4];
     bias_tiles<2>(y, net.w32 + oB3, kOut, q);
     hidden_product<2>(y, h, Bs + fW3 * 32, lane);

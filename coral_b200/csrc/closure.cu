@@ -533,7 +533,7 @@ __global__ void __launch_bounds__(kTrainThreads, 1) k_closure_train(NetDev net, 
   }
   grad += (size_t)(blockIdx.x % kGradBuckets) * kNParam;
   const float inv = 1.0f / (float)npts;
-  float l = 0.0f;
+  double l = 0.0;  // (FP32 within a point only: a chain over a CTA's tiles would grow with the batch)
   for (long long p0 = (long long)blockIdx.x * kTP; p0 < npts; p0 += (long long)gridDim.x * kTP) {
     __syncthreads();  // the weights are in; the previous points are done with
     const bool ok = p0 + pt < npts;
@@ -578,15 +578,17 @@ __global__ void __launch_bounds__(kTrainThreads, 1) k_closure_train(NetDev net, 
           if (part + 4 * m < kOut) y[m] = fmaf(sm[sW3 + (part + 4 * m) * kHid + k], x, y[m]);
       }
       const float* tg = targets + snap * kOut * npoint + lin;
+      float lp = 0.0f;
 #pragma unroll
       for (int m = 0; m < 3; ++m) {
         const int o = part + 4 * m;
         if (o < kOut) {
           const float d = ok ? y[m] - tg[(long long)o * npoint] / net.out_scale[o] : 0.0f;
-          l += d * d;
+          lp += d * d;
           sm[sY + o * kTR + pt] = 2.0f * d * inv;
         }
       }
+      l += (double)lp;
     }
     __syncthreads();
     {  // dW3, db3
@@ -623,7 +625,7 @@ __global__ void __launch_bounds__(kTrainThreads, 1) k_closure_train(NetDev net, 
     if (part == 0) atomicAdd(grad + oB0 + pt, row_sum(sm + sH1 + pt * kTR));
   }
   for (int o = 16; o > 0; o >>= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
-  if ((t & 31) == 0 && l != 0.0f) atomicAdd(loss, (double)l * inv);
+  if ((t & 31) == 0 && l != 0.0) atomicAdd(loss, l * inv);
 }
 
 __device__ __forceinline__ float grad_sum(const float* g, int i) {

@@ -125,9 +125,17 @@ __device__ __forceinline__ void split3(float a, float b, unsigned& p0, unsigned&
   b -= __uint_as_float(p1 & 0xffff0000u);
   p2 = pack2(a, b);
 }
-// the same for values that may be infinite or round to it (the rests are then zero)
-__device__ __forceinline__ void split3_inf(float a, float b, unsigned& p0, unsigned& p1, unsigned& p2) {
-  split3(a, b, p0, p1, p2);
+// the same for any value: the first plane is cut off, not rounded, so that finite
+// values up to the largest FP32 stay finite (rounding takes those above 3.396e38 to
+// infinity, and two of opposite sign to NaN); infinities have zero rests
+__device__ __forceinline__ void split3_any(float a, float b, unsigned& p0, unsigned& p1, unsigned& p2) {
+  p0 = __byte_perm(__float_as_uint(a), __float_as_uint(b), 0x7632);
+  a -= __uint_as_float(p0 << 16);
+  b -= __uint_as_float(p0 & 0xffff0000u);
+  p1 = pack2(a, b);
+  a -= __uint_as_float(p1 << 16);
+  b -= __uint_as_float(p1 & 0xffff0000u);
+  p2 = pack2(a, b);
   const unsigned keep = ((p0 & 0x7f80u) == 0x7f80u ? 0u : 0xffffu) | ((p0 & 0x7f800000u) == 0x7f800000u ? 0u : 0xffff0000u);
   p1 &= keep;
   p2 &= keep;
@@ -213,9 +221,9 @@ __device__ __forceinline__ void input_planes(unsigned (&a)[3][4], const PointRow
                                              const F* f, float sc, int q) {
 #pragma unroll
   for (int i = 0; i < 2; ++i) {
-    split3_inf(point_input<KS, 0>(r[i], z[i], f, sc, q), point_input<KS, 1>(r[i], z[i], f, sc, q), a[0][i], a[1][i],
+    split3_any(point_input<KS, 0>(r[i], z[i], f, sc, q), point_input<KS, 1>(r[i], z[i], f, sc, q), a[0][i], a[1][i],
                a[2][i]);
-    split3_inf(point_input<KS, 2>(r[i], z[i], f, sc, q), point_input<KS, 3>(r[i], z[i], f, sc, q), a[0][2 + i],
+    split3_any(point_input<KS, 2>(r[i], z[i], f, sc, q), point_input<KS, 3>(r[i], z[i], f, sc, q), a[0][2 + i],
                a[1][2 + i], a[2][2 + i]);
   }
 }

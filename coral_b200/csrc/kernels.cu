@@ -31,14 +31,6 @@ constexpr int kQC = 5;   // quadratic variables per FFT batch, forward z pass (o
                          // butterfly per thread at NZAA = 288)
 constexpr int kPadRt = 2;  // line stride N + 2 of the x / y passes with run-time plans
 constexpr int kThreads = 256;
-// FFT plans of the time-step transforms (fft.cuh plan_of): the x passes and the
-// fused z passes use the two-pass plans (576 = 24 x 24, 288 = 18 x 16); the y
-// passes, whose first pass gathers its inputs (spectral build, strided
-// coefficients), keep the three-pass plans with their shorter per-thread load
-// chains (measured at 384^2 x 192)
-constexpr int kPlanHot = 1;
-constexpr int kPlanY = 0;
-constexpr int kPlanFZ = 2;  // separate forward z pass
 // x / y passes: threads per CTA for nl lines of a compiled length N, the most
 // that any pass keeps busy, rounded up to whole warps: one butterfly per thread,
 // of radix 2, 3 and 4 as many as make 8 or 9 elements (one radix-3 butterfly each
@@ -428,7 +420,7 @@ __host__ __device__ constexpr int z_threads(int N, int nl, int pv = kPlanHot) {
 // via an NZAA-point complex FFT (two columns per FFT); also the CFL maxima of
 // compute_cfl_based_timestep (marching.f90:219-238) for the first three full variables
 // ------------------------------------------------------------------------------
-#define kThreadsIZ z_threads(NF, kXB3 / 2, kPlanY)
+#define kThreadsIZ z_threads(NF, kXB3 / 2, kPlanInvZ)
 template <int NF>
 __global__ void __launch_bounds__(kThreadsIZ, hot_min_blocks(kThreadsIZ)) k_inv_z(Dims d, const double* Y2, double* phys,
                                                                                  FftPlan pz, const double2* dct_tw,
@@ -438,7 +430,7 @@ __global__ void __launch_bounds__(kThreadsIZ, hot_min_blocks(kThreadsIZ)) k_inv_
   extern __shared__ double2 sm[];
   __shared__ double red[NT / 32];
   const int f = blockIdx.x, x0 = blockIdx.y * kXB3, y = blockIdx.z;
-  const int N = NF ? NF : d.NZA, NP = kXB3 / 2, LZ = NF ? line_len(NF, kPlanY, false) : N;
+  const int N = NF ? NF : d.NZA, NP = kXB3 / 2, LZ = NF ? line_len(NF, kPlanInvZ, false) : N;
   double2* A = sm;
   double2* B = sm + NP * LZ;  // runtime plan only
   const double* src0 = Y2 + (((size_t)f * d.NYA + y) * d.NXA + x0) * d.NZ;
@@ -455,7 +447,7 @@ __global__ void __launch_bounds__(kThreadsIZ, hot_min_blocks(kThreadsIZ)) k_inv_
     const double2 vb = cmul(w, make_double2(b0, -b1));
     return make_double2(va.x - vb.y, va.y + vb.x);
   };
-  const double2* R = fft_lines_ld<NF, true, NT, kXB3 / 2, false, kPlanY>(A, B, NP, LZ, pz, ld);
+  const double2* R = fft_lines_ld<NF, true, NT, kXB3 / 2, false, kPlanInvZ>(A, B, NP, LZ, pz, ld);
   double mx = 0.0;
   const int which = (f < 3) ? f : -1;
   for (int idx = threadIdx.x; idx < NP * N; idx += blockDim.x) {
@@ -3250,14 +3242,6 @@ int resident_by_smem(K kernel, size_t bytes) {
 }  // namespace
 
 // ---- launchers ----------------------------------------------------------------
-// Each transform kernel is instantiated for every length 3 N / 2 of a grid (N a
-// multiple of 4, so 2^a 3^b multiples of 6) from 24 to 576; other lengths use the
-// runtime plan, whose radix 2-4 passes ping-pong through shared memory
-// (108 x 64 x 72 modes, run-time against compiled plans, per step: fused z pass 0.43
-// and 0.19 ms, forward x 0.226 and 0.093, inverse x 0.119 and 0.058).
-#define CORAL_FFT_LENGTHS(X) \
-  X(24) X(36) X(48) X(54) X(72) X(96) X(108) X(144) X(162) X(192) X(216) X(288) X(324) X(384) X(432) X(486) X(576)
-
 template <template <int> class L, typename... Args>
 void dispatch_len(int n, Args&&... args) {
   switch (n) {
@@ -3338,7 +3322,7 @@ template <int NF>
 struct InvZ {
   static void run(const Dims& d, int nf, const double* Y2, double* phys, const FftPlan& pz, const double2* dct_tw,
                   const double* wz, unsigned long long* cfl_bits, cudaStream_t s) {
-    size_t sm = (NF ? 1 : 2) * (kXB3 / 2) * (size_t)(NF ? line_len(NF, kPlanY, false) : d.NZA) * sizeof(double2);
+    size_t sm = (NF ? 1 : 2) * (kXB3 / 2) * (size_t)(NF ? line_len(NF, kPlanInvZ, false) : d.NZA) * sizeof(double2);
     set_smem(k_inv_z<NF>, sm);
     dim3 g(nf, (d.NXA + kXB3 - 1) / kXB3, d.NYA);
     k_inv_z<NF><<<g, kThreadsIZ, sm, s>>>(d, Y2, phys, pz, dct_tw, wz, cfl_bits);

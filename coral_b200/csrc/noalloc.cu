@@ -22,11 +22,8 @@ using namespace coral;
 namespace {
 
 constexpr size_t kScratchBytes = size_t(64) << 20;  // 64 MiB, the stated maximum
-constexpr int kMaxTableLen = 4096;                  // 6 tables of < 2 N entries fit kTableBytes
 constexpr int kMaxModes = 1 << 16;                  // per direction, checked first
-// beyond the stated maximum: the pass tables of the compiled FFT plans (two per axis)
-constexpr size_t kTableBytes = size_t(1) << 20;
-__device__ __align__(256) unsigned char g_scratch[kScratchBytes + kTableBytes];
+__device__ __align__(256) unsigned char g_scratch[kScratchBytes];
 
 // The device address of g_scratch, looked up once per device and CUDA context
 // with that device current (in host code the array's name is only a stand-in
@@ -92,14 +89,13 @@ void* scratch_address() {
   return slot.addr;
 }
 
-// The twiddle tables of a call in one launch: per axis exp(-2 pi i k / N), k < N,
-// and the pass tables of the compiled plans (entries of the former); for z also
-// exp(-i pi k / 2N), the rotation of the FFT-based Chebyshev transform
+// The twiddle tables of a call in one launch.  Per axis the one its pass reads: for a
+// compiled length the plan's pass table (pass_tw_len(N, pv) = N minus the first radix
+// entries), else exp(-2 pi i k / N), k < N; for z also exp(-i pi k / 2N), the rotation
+// of the FFT-based Chebyshev transform.
 struct Tables {
-  int N[3];
+  int N[3], pv[3], len[3];  // pv: plan variant of a compiled length, -1: run-time plan
   double2* tw[3];
-  double2* tws[3][2];
-  int len[3][2];
   double2* dct;
 };
 __device__ __forceinline__ double2 unit_root(double a, int N) {  // exp(-i pi a / N)
@@ -114,21 +110,12 @@ __global__ void k_twiddles(Tables t, int total) {
     bool done = false;
 #pragma unroll
     for (int ax = 0; ax < 3; ++ax) {
-      const int N = t.N[ax];
-      if (!done && k < N) {
-        t.tw[ax][k] = unit_root(2.0 * (double)k, N);
+      const int N = t.N[ax], n = t.len[ax];
+      if (!done && k < n) {
+        t.tw[ax][k] = unit_root(2.0 * (double)(t.pv[ax] < 0 ? k : pass_tw_index(N, t.pv[ax], k)), N);
         done = true;
       }
-      k -= done ? 0 : N;
-#pragma unroll
-      for (int pv = 0; pv < 2; ++pv) {
-        const int n = t.len[ax][pv];
-        if (!done && k < n) {
-          t.tws[ax][pv][k] = unit_root(2.0 * (double)pass_tw_index(N, pv, k), N);
-          done = true;
-        }
-        k -= done ? 0 : n;
-      }
+      k -= done ? 0 : n;
     }
     if (!done) t.dct[k] = unit_root(0.5 * (double)k, t.N[2]);
   }
@@ -198,21 +185,22 @@ extern "C" int coral_spec_to_phys_noalloc(int NX, int NY, int NZ, const double* 
     // then the y pass fills Y1, the x pass fills Y2), so nothing needs clearing
     const Dims d{NXH, NYA, NXA, NZ, NZA};
     FftPlan pl[3] = {plan_in(NYA, ty), plan_in(NXA, tx), plan_in(NZA, tz)};
-    Tables tab{{NYA, NXA, NZA}, {ty, tx, tz}, {}, {}, td};
-    size_t at = kScratchBytes;
-    for (int ax = 0; ax < 3; ++ax)
-      for (int pv = 0; pv < 2; ++pv) {
-        // (axes longer than the compiled lengths take run-time plans, no pass tables)
-        tab.len[ax][pv] = tab.N[ax] <= kMaxTableLen ? pass_tw_len(tab.N[ax], pv) : 0;
-        pl[ax].tws[pv] = tab.tws[ax][pv] = reinterpret_cast<double2*>(base + at);
-        at += up256((size_t)tab.len[ax][pv] * sizeof(double2));
+    Tables tab{{NYA, NXA, NZA}, {kPlanY, kPlanHot, kPlanInvZ}, {}, {ty, tx, tz}, td};
+    int total = NZA;
+    for (int ax = 0; ax < 3; ++ax) {
+      if (compiled_length(tab.N[ax])) {
+        tab.len[ax] = pass_tw_len(tab.N[ax], tab.pv[ax]);  // < N: in the N-entry table's place
+        pl[ax].tws[tab.pv[ax]] = tab.tw[ax];
+      } else {
+        tab.len[ax] = tab.N[ax];
+        tab.pv[ax] = -1;
       }
-    int total = tab.N[2];
-    for (int ax = 0; ax < 3; ++ax) total += tab.N[ax] + tab.len[ax][0] + tab.len[ax][1];
+      total += tab.len[ax];
+    }
     k_twiddles<<<std::min((total + 63) / 64, 592), 64, 0, s>>>(tab, total);
     const FftPlan &py = pl[0], &px = pl[1], &pz = pl[2];
     launch_inv_y(d, 1, nullptr, StateSet{}, reinterpret_cast<const double2*>(spec), nullptr, nullptr, Y1, py, s);
-    launch_inv_x(d, 1, Y1, Y2, px, s);
+    launch_inv_x(d, 1, Y1, Y2, px, s, kPlanHot);
     launch_inv_z(d, 1, Y2, phys, pz, td, nullptr, nullptr, s);
     // nothing was pending at entry, so an error now comes from these launches
     cudaError_t e = cudaGetLastError();

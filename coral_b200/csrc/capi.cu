@@ -74,6 +74,9 @@ bool smooth23(int n) {
   return n == 1;
 }
 
+// factors up to this size keep their packed form in a buffer of its own
+constexpr size_t kStageBytes = size_t(64) << 20;
+
 struct KSys {
   SystemOps ops;
   DevEll M, L, NL;
@@ -99,8 +102,8 @@ struct KSys {
   int *slot = nullptr, *lane_sid = nullptr, *unit_sid = nullptr;
   unsigned char *row_neg = nullptr, *col_neg = nullptr;
   unsigned long long* cmask = nullptr;
-  double *lpack = nullptr, *upack = nullptr;
-  int fac_chunk = 1;  // groups of each class in abr (block layout)
+  double *pack = nullptr, *stage = nullptr;
+  int nstage = 0;
   uint4* finfo = nullptr;
   uint4* binfo = nullptr;
   int* ptot = nullptr;
@@ -854,20 +857,28 @@ void setup(coral_handle* h, const std::string& eqs, const std::string& pars, con
       k.unit_sid = mem.upload(unit_sid);
       k.row_neg = mem.upload(k.ops.row_neg);
       k.col_neg = mem.upload(k.ops.col_neg);
-      const size_t ng = 2 * (size_t)k.ngrp, cols = ng * k.Tc, kv = (size_t)k.kl_s + k.ku_s;
-      // the factorisation's workspace: all groups, or a 16th of them where that would
-      // take more than a quarter of the memory left (the packed factors, as large,
-      // and the transforms' buffers are still to come)
-      const size_t per_group = 2 * (size_t)k.Tc * k.ldab_s * k.upw;
-      size_t mfree = 0, mtotal = 0;
-      CK(cudaMemGetInfo(&mfree, &mtotal));
-      k.fac_chunk = std::max(k.ngrp, 1);
-      if (per_group * k.ngrp * sizeof(double) > mfree / 4) k.fac_chunk = (k.ngrp + 15) / 16;
-      if (const char* e = std::getenv("CORAL_FACTOR_CHUNK"); e && std::atoi(e) > 0)
-        k.fac_chunk = std::min(k.fac_chunk, std::atoi(e));
-      k.abr = mem.get<double>(per_group * k.fac_chunk);
-      k.lpack = mem.get<double>(cols * std::max(k.kl_s, 1) * k.upw);
-      k.upack = mem.get<double>(cols * (kv + 1) * k.upw);
+      const size_t ng = 2 * (size_t)k.ngrp, cols = ng * k.Tc;
+      // Factors and their packed form: in two buffers where together they take about
+      // what one factorisation a system does (units that two systems share) or are
+      // small; else the packed form goes back into the factors' own place, kStageBytes or
+      // a 16th at a time, so that a handle holds its factors once (rotating recipe,
+      // two buffers | in place: 192^2 x 96 8.88 | 6.31 GB and 6.9 | 7.5 ms a
+      // factorisation, 288^2 x 144 30.1 | 21.4 GB and 21.3 | 23.2 ms).
+      const size_t per_group = 2 * (size_t)k.Tc * k.ldab_s * k.upw, bytes = per_group * k.ngrp * sizeof(double);
+      const size_t room = (size_t)h->nact * 2 * k.Tc * k.ldab_s * sizeof(double);
+      k.abr = mem.get<double>(per_group * k.ngrp);
+      int groups = k.ngrp;
+      if (2 * bytes > room + room / 8 && bytes > kStageBytes)
+        groups = std::max((k.ngrp + 15) / 16, (int)(kStageBytes / (per_group * sizeof(double))));
+      if (const char* e = std::getenv("CORAL_FACTOR_CHUNK"); e && std::atoi(e) > 0) groups = std::min(k.ngrp, std::atoi(e));
+      double* second = mem.get<double>(per_group * groups);
+      if (groups == k.ngrp) {
+        k.pack = second;
+      } else {
+        k.pack = k.abr;
+        k.stage = second;
+        k.nstage = groups;
+      }
       k.dpiv = mem.get<unsigned char>(cols * k.upw);
       k.work2 = mem.get<double2>(cols * 32);
       k.cmask = mem.get<unsigned long long>(2 * (size_t)k.Tc);
@@ -1228,8 +1239,7 @@ SolveArgs make_solve_args(coral_handle* h, KSys& k, int i, double dt) {
   sa.slot = k.slot;
   sa.lane_sid = k.lane_sid;
   sa.row_neg = k.row_neg;
-  sa.lpack = k.lpack;
-  sa.upack = k.upack;
+  sa.pack = k.pack;
   sa.finfo = k.finfo;
   sa.binfo = k.binfo;
   sa.ptot = k.ptot;
@@ -1542,11 +1552,10 @@ void factorize(coral_handle* h, double dt) {
     fa.window = h->tune.factor_window;
     fa.upw = k.upw;
     fa.ngrp = k.ngrp;
-    fa.g0 = 0;
-    fa.gn = k.fac_chunk;
     fa.cmask = k.cmask;
-    fa.lpack = k.lpack;
-    fa.upack = k.upack;
+    fa.pack = k.pack;
+    fa.stage = k.stage;
+    fa.nstage = k.nstage;
     fa.finfo = k.finfo;
     fa.binfo = k.binfo;
     fa.ptot = k.ptot;

@@ -265,7 +265,7 @@ struct SolveArgs {
   // (kx, ky) and (kx, -ky) when the recipe has the ky mirror symmetry; a group is
   // upw units (16 with the symmetry, else 32) of one class, 32 lanes = the
   // right-hand sides of its units (mirror symmetry: lanes 16-31 are the -ky
-  // systems).  Group G = class * ngrp + g; packed factors lpack / upack (see
+  // systems).  Group G = class * ngrp + g; packed factors pack (see
   // k_pack), pivots dpiv[(G Tc + j) upw + unit], right-hand sides and solutions
   // work2[(G Tc + j) 32 + lane].
   double2* work2;        // null: warp-per-system layouts
@@ -273,12 +273,11 @@ struct SolveArgs {
   const int* slot;       // [kx*NYA+ky] 32 g + lane of an active system, bit 30: its -ky partner's unit
   const int* lane_sid;   // [32 ngrp] kx*NYA+ky of a lane's system, -1 = none
   const unsigned char* row_neg;  // [T] rows negated for the -ky system of a unit
-  const double* lpack;
-  const double* upack;
+  const double* pack;
   const uint4* finfo;    // [2 Tc] per class and column: its L record (k_pack_info)
   const uint4* binfo;    // [2 Tc] per class and step of the backward sweep: its U record, variable column
                          // and signs
-  const int* ptot;       // [4] rows per group of lpack and upack: (class 0, class 1) of each
+  const int* ptot;       // [4] rows per group of the L and of the U records: (class 0, class 1) of each
   // operator-stationary K_std (null tile_win: k_kstd_out): rows in tiles of
   // kTileRows; tile_win[2 tile + .] = (start, width) of the solution columns the
   // tile's rows of L touch; Lw = L with its columns relative to that window
@@ -337,15 +336,15 @@ struct FactorArgs {
   const int* col_pos;    // [T] class position of a variable column
   // block layout (see SolveArgs::work2; act_list then lists the units' systems,
   // nact their number): factors abr[((G Tc + j) ldab + r) upw + unit], packed for
-  // the substitution into lpack / upack by k_pack
+  // the substitution by k_pack
   int tpb, upw, ngrp;
-  // abr holds the groups g0 .. g0 + gn - 1 of each class (all, or a chunk of them:
-  // see launch_factor_real)
-  int g0, gn;
   int window;            // block layout: 1 shared-memory band window, 0 in place in global memory
   unsigned long long* cmask;  // [2 Tc] per class and column, the band rows nonzero in any unit
-  double* lpack;
-  double* upack;
+  // packed factors: a buffer of their own as large as abr (stage null), or abr itself,
+  // through stage, which holds nstage groups of each class at a time
+  double* pack;
+  double* stage;
+  int nstage;
   uint4* finfo;
   uint4* binfo;
   int* ptot;

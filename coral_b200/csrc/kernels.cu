@@ -1617,9 +1617,9 @@ struct TpbBlock {
 };
 __device__ __forceinline__ bool tpb_block(const FactorArgs& a, int b, TpbBlock& t) {
   const int G = b / a.upw, lane = b - G * a.upw;
-  if (G >= a.ncls * a.gn) return false;
-  t.cls = G / a.gn;
-  const int g = a.g0 + G - t.cls * a.gn;
+  if (G >= a.ncls * a.ngrp) return false;
+  t.cls = G / a.ngrp;
+  const int g = G - t.cls * a.ngrp;
   t.unit = g * a.upw + lane;
   t.F = a.abr + (size_t)G * a.Tc * a.ldab * a.upw + lane;
   t.P = a.dpiv + ((size_t)t.cls * a.ngrp + g) * a.Tc * a.upw + lane;
@@ -1870,7 +1870,7 @@ __global__ void __launch_bounds__(256) k_mask_cols(FactorArgs a) {
   const int G = blockIdx.x, j = blockIdx.y * 8 + w;
   const int T = a.Tc, ldab = a.ldab;
   if (j >= T) return;
-  const int cls = G / a.gn, u0 = (a.g0 + G - cls * a.gn) * a.upw;
+  const int cls = G / a.ngrp, u0 = (G - cls * a.ngrp) * a.upw;
   const bool ok = lane < a.upw && u0 + lane < a.nact;
   const double* F = a.abr + ((size_t)G * T + j) * ldab * a.upw + (ok ? lane : 0);
   unsigned long long bits = 0;
@@ -1881,13 +1881,13 @@ __global__ void __launch_bounds__(256) k_mask_cols(FactorArgs a) {
   if (lane == 0 && bits) atomicOr(a.cmask + (size_t)cls * T + j, bits);
 }
 // The records of the substitution from cmask, one warp per class.  A factor row
-// is upw doubles (one entry of every unit of a group).  Forward: column j's
-// record in lpack is its L rows i (band row kl+ku+1+i) that are nonzero in some
-// unit.  Backward: step k handles row j = Tc-1-k; its record in upack is the
-// reciprocal diagonal (row 0) and the entries (j, j+i) (row i) that are nonzero
-// in some unit.  Rows in increasing i.
-//   finfo[k] = first row, mask of the rows held
-//   binfo[k] = first row, mask of the rows held, variable column (-1 = padding),
+// is upw doubles (one entry of every unit of a group).  A group's rows: first its L
+// records, forward, column j's being its L rows i (band row kl+ku+1+i) that are
+// nonzero in some unit; then its U records, step k of the backward sweep handling
+// row j = Tc-1-k: the reciprocal diagonal (row 0) and the entries (j, j+i) (row i)
+// that are nonzero in some unit.  Rows in increasing i.
+//   finfo[k] = first row (of the L records), mask of the rows held
+//   binfo[k] = first row (of the U records), mask of the rows held, variable column (-1 = padding),
 //              bit 0 colflip, bit 1 col_neg
 // ptot: rows per group.
 __global__ void __launch_bounds__(32) k_pack_info(FactorArgs a) {
@@ -1930,24 +1930,25 @@ __global__ void __launch_bounds__(32) k_pack_info(FactorArgs a) {
     a.ptot[2 + cls] = base[1];
   }
 }
-// first row of group G's records in lpack (q = 0) or upack (q = 1)
-__device__ __forceinline__ size_t pack_base(const int* ptot, int q, int cls, int g, int ngrp) {
-  const int t0 = ptot[2 * q], t1 = ptot[2 * q + 1];
-  return cls == 0 ? (size_t)g * t0 : (size_t)ngrp * t0 + (size_t)g * t1;
+// first row of group G's L (q = 0) or U (q = 1) records: a group starts where its
+// factors do in abr (Tc ldab rows, more than all of its records)
+__device__ __forceinline__ size_t pack_base(const int* ptot, int q, int cls, size_t G, int Tc, int ldab) {
+  return G * Tc * ldab + (q ? ptot[cls] : 0);
 }
-// The band factors copied into the records: one warp per (group, column).  The
-// substitution then reads two linear streams that hold only what it needs.
-__global__ void __launch_bounds__(256) k_pack(FactorArgs a) {
+// The band factors of the groups g0 .. g0 + gn - 1 of each class copied into records in
+// out (group cls gn + g - g0 there): one warp per (group, column).  The substitution
+// then reads two linear streams that hold only what it needs.
+__global__ void __launch_bounds__(256) k_pack(FactorArgs a, double* out, int g0, int gn) {
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int G = blockIdx.x, k = blockIdx.y * 8 + w;
+  const int k = blockIdx.y * 8 + w;
   const int T = a.Tc, kv = a.kl + a.ku, ldab = a.ldab, RW = a.upw;
   if (k >= T) return;
-  const int cls = G / a.gn, g = a.g0 + G - cls * a.gn;
-  const double* F = a.abr + (size_t)G * T * ldab * RW;
+  const int cls = blockIdx.x / gn, g = g0 + blockIdx.x - cls * gn;
+  const double* F = a.abr + ((size_t)cls * a.ngrp + g) * T * ldab * RW;
   const int half = lane / RW, ln = lane - half * RW, per = 32 / RW;  // rows a warp copies at a time
   {
     const uint4 fi = a.finfo[(size_t)cls * T + k];
-    double* dst = a.lpack + (pack_base(a.ptot, 0, cls, g, a.ngrp) + fi.x) * RW;
+    double* dst = out + (pack_base(a.ptot, 0, cls, blockIdx.x, T, ldab) + fi.x) * RW;
     const int n = __popc(fi.y);
     for (int r = half; r < n; r += per) {
       const int i = __fns(fi.y, 0, r + 1);  // the (r + 1)-th set bit
@@ -1956,13 +1957,23 @@ __global__ void __launch_bounds__(256) k_pack(FactorArgs a) {
   }
   {
     const uint4 bi = a.binfo[(size_t)cls * T + k];
-    double* dst = a.upack + (pack_base(a.ptot, 1, cls, g, a.ngrp) + bi.x) * RW;
+    double* dst = out + (pack_base(a.ptot, 1, cls, blockIdx.x, T, ldab) + bi.x) * RW;
     const int j = T - 1 - k, n = __popc(bi.y);
     for (int r = half; r < n; r += per) {
       const int i = __fns(bi.y, 0, r + 1);
       dst[(size_t)r * RW + ln] = F[((size_t)(j + i) * ldab + kv - i) * RW + ln];
     }
   }
+}
+// The staged records of those groups over their factors; blockIdx.y takes a part of a
+// group's rows.
+__global__ void __launch_bounds__(256) k_pack_back(FactorArgs a, int g0, int gn) {
+  const int cls = blockIdx.x / gn, g = g0 + blockIdx.x - cls * gn;
+  const size_t group = (size_t)a.Tc * a.ldab * a.upw / 2;  // in 16-byte words
+  const int n = (a.ptot[cls] + a.ptot[2 + cls]) * a.upw / 2;
+  const double2* src = reinterpret_cast<const double2*>(a.stage) + blockIdx.x * group;
+  double2* dst = reinterpret_cast<double2*>(a.abr) + ((size_t)cls * a.ngrp + g) * group;
+  for (int e = blockIdx.y * 256 + threadIdx.x; e < n; e += gridDim.y * 256) dst[e] = src[e];
 }
 
 // ------------------------------------------------------------------------------
@@ -2076,7 +2087,7 @@ __device__ __forceinline__ void subst_group(const SolveArgs& a, int b, unsigned 
   {
     constexpr int U = 4;
     constexpr int NA = KL < 6 ? KL : 6;       // L rows handled without a test
-    const char* L = reinterpret_cast<const char*>(a.lpack + pack_base(a.ptot, 0, cls, g, a.ngrp) * UPW);
+    const char* L = reinterpret_cast<const char*>(a.pack + pack_base(a.ptot, 0, cls, G, T, a.ldab) * UPW);
     const unsigned char* P = a.dpiv + (size_t)G * T * UPW;
     const int nc = T - 1;  // columns
     RecordBlock info(a.finfo + (size_t)cls * T, nc, lane);
@@ -2183,7 +2194,7 @@ __device__ __forceinline__ void subst_group(const SolveArgs& a, int b, unsigned 
     constexpr int NA = 12;   // U rows handled without a test (row 0 the diagonal)
     constexpr int CB = kRowGroup;
     static_assert(NA % CB == 0 && NA <= KV, "groups");
-    const char* Up = reinterpret_cast<const char*>(a.upack + pack_base(a.ptot, 1, cls, g, a.ngrp) * UPW);
+    const char* Up = reinterpret_cast<const char*>(a.pack + pack_base(a.ptot, 1, cls, G, T, a.ldab) * UPW);
     double2* out = a.out + (size_t)(sid >= 0 ? sid : 0) * a.T;
     bool bad = false;
     RecordBlock info(a.binfo + (size_t)cls * T, T, lane);
@@ -3784,9 +3795,9 @@ void launch_solve_real(const SolveArgs& a, const NLArgs& n, cudaStream_t s) {
   launch_subst(a, s);
   launch_kstd_out(a, s);
 }
-// the band factorisation of the groups that a.abr holds
+// Block layout: the union masks need every group's factors before any is packed.
 static void launch_factor_blocks(const FactorArgs& a, cudaStream_t s) {
-  const int nb = a.ncls * a.gn * a.upw;
+  const int nb = a.ncls * a.ngrp * a.upw;
   const size_t sm = (size_t)(a.kl + 1) * (a.kl + a.ku + 1) * 32 * sizeof(double);
   cudaMemsetAsync(a.abr, 0, (size_t)nb * a.Tc * a.ldab * sizeof(double), s);
   if (a.window && a.kl <= kFacKl && a.kl + a.ku <= kFacKv) {
@@ -3803,28 +3814,25 @@ static void launch_factor_blocks(const FactorArgs& a, cudaStream_t s) {
   } else {
     k_factor_tpb<<<(nb + kTpbThreads - 1) / kTpbThreads, kTpbThreads, 0, s>>>(a);
   }
+  const auto cols = [&](int gn) { return dim3(a.ncls * gn, (a.Tc + 7) / 8); };
+  cudaMemsetAsync(a.cmask, 0, (size_t)a.ncls * a.Tc * sizeof(unsigned long long), s);
+  k_mask_cols<<<cols(a.ngrp), 256, 0, s>>>(a);
+  k_pack_info<<<a.ncls, 32, 0, s>>>(a);
+  if (!a.stage) {
+    k_pack<<<cols(a.ngrp), 256, 0, s>>>(a, a.pack, 0, a.ngrp);
+    return;
+  }
+  for (int g0 = 0; g0 < a.ngrp; g0 += a.nstage) {
+    const int gn = std::min(a.nstage, a.ngrp - g0);
+    k_pack<<<cols(gn), 256, 0, s>>>(a, a.stage, g0, gn);
+    // as many CTAs as hold the chip, at least one a group
+    k_pack_back<<<dim3(a.ncls * gn, std::max(1, 8 * 148 / (a.ncls * gn))), 256, 0, s>>>(a, g0, gn);
+  }
 }
-// Block layout: the union masks need every group's factors before any is packed.
-// With a workspace of all groups (chunk = ngrp) each group is factored once; with a
-// smaller one, where memory is short, twice: for the masks, then for the packing.
-void launch_factor_real(const FactorArgs& full, cudaStream_t s) {
-  FactorArgs a = full;
+void launch_factor_real(const FactorArgs& a, cudaStream_t s) {
   if (a.nact <= 0) return;
   if (a.tpb) {
-    const int chunk = full.gn;
-    const auto rows = [&](int gn) { return dim3(full.ncls * gn, (full.Tc + 7) / 8); };
-    cudaMemsetAsync(a.cmask, 0, (size_t)a.ncls * a.Tc * sizeof(unsigned long long), s);
-    for (a.g0 = 0; a.g0 < a.ngrp; a.g0 += chunk) {
-      a.gn = std::min(chunk, a.ngrp - a.g0);
-      launch_factor_blocks(a, s);
-      k_mask_cols<<<rows(a.gn), 256, 0, s>>>(a);
-    }
-    k_pack_info<<<a.ncls, 32, 0, s>>>(a);
-    for (a.g0 = 0; a.g0 < a.ngrp; a.g0 += chunk) {
-      a.gn = std::min(chunk, a.ngrp - a.g0);
-      if (chunk < a.ngrp) launch_factor_blocks(a, s);
-      k_pack<<<rows(a.gn), 256, 0, s>>>(a);
-    }
+    launch_factor_blocks(a, s);
     return;
   }
   k_factor_real<<<dim3((a.nact + kWPB - 1) / kWPB, a.ncls), kWPB * 32, 0, s>>>(a);

@@ -92,10 +92,8 @@ struct KSys {
   int* info;
   // class split of the real-scaled solve (SystemOps::ncls == 2); when unsplit:
   // ncls = 1, Tc = T, the band (kl_s, ku_s, ldab_s) of the whole system, work = aux
-  int ncls = 1, Tc = 0, kl_s = 0, ku_s = 0, ldab_s = 0, wst = 0;
+  int ncls = 1, Tc = 0, kl_s = 0, ku_s = 0, ldab_s = 0;
   int *row_pos = nullptr, *col_pos = nullptr, *cls_row = nullptr, *cls_col = nullptr;
-  unsigned char* colflip_cls = nullptr;
-  DevEll Lp;
   // block layout of a split system (SolveArgs::work2): factorisation units, each
   // shared by the (kx, ky) and (kx, -ky) systems of a recipe with that symmetry
   int upw = 32, ngrp = 0, nunit = 0;
@@ -725,10 +723,7 @@ void setup(coral_handle* h, const std::string& eqs, const std::string& pars, con
     k.kl_s = k.kl;
     k.ku_s = k.ku;
     k.ldab_s = k.ldab;
-    k.wst = k.T;
     k.work = k.aux;
-    k.Lp = k.L;
-    k.colflip_cls = k.colflip;
     if (k.real && k.ops.ncls == 2 && k.ops.kl_cls <= 15 && k.ops.kl_cls + k.ops.ku_cls <= 31 &&
         std::getenv("CORAL_NO_CLASS_SPLIT") == nullptr) {
       k.ncls = 2;
@@ -746,13 +741,6 @@ void setup(coral_handle* h, const std::string& eqs, const std::string& pars, con
         for (int t = 0; t < k.T; ++t) cc[k.ops.col_cls_pos[t]] = t;
         k.cls_col = mem.upload(cc);
       }
-      std::vector<unsigned char> cf(2 * (size_t)k.Tc, 0);
-      for (int t = 0; t < k.T; ++t) cf[k.ops.col_cls_pos[t]] = k.ops.col_flip[t];
-      k.colflip_cls = mem.upload(cf);
-      EllOp lp = k.ops.L;
-      for (int& c : lp.col)
-        if (c >= 0) c = k.ops.col_cls_pos[c];
-      k.Lp = upload_ell(mem, lp);
     }
     if (k.ncls == 2) {
       // K_std in tiles of kTileRows rows: per tile the window of solution columns
@@ -1228,11 +1216,7 @@ SolveArgs make_solve_args(coral_handle* h, KSys& k, int i, double dt) {
   sa.colflip = k.colflip;
   sa.ncls = k.ncls;
   sa.Tc = k.Tc;
-  sa.wst = k.wst;
   sa.row_pos = k.row_pos;
-  sa.col_pos = k.col_pos;
-  sa.colflip_cls = k.colflip_cls;
-  sa.Lp = k.Lp;
   sa.work2 = k.work2;
   sa.upw = k.upw;
   sa.ngrp = k.ngrp;
@@ -1258,7 +1242,7 @@ SolveArgs make_solve_args(coral_handle* h, KSys& k, int i, double dt) {
   {
     const int kv = sa.kl + sa.ku;
     const int u_rows = (kv + 2) & ~1, l_rows = ((kv + 1 + sa.kl + 1) & ~1) - ((kv + 1) & ~1);
-    sa.ring_cols = k.ncls * std::max(u_rows, l_rows);
+    sa.ring_cols = std::max(u_rows, l_rows);
   }
   return sa;
 }

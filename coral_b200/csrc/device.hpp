@@ -252,15 +252,9 @@ struct SolveArgs {
   int ring_cols;         // doubles per column slot of the solve's shared-memory ring
   int nact;              // active systems (factor slots)
   const int* act_list;   // [nact] kx*NYA+ky of each factor slot
-  // class split (SystemOps::ncls == 2): factors of both classes interleaved per
-  // column (column stride ncls*ldab), kl/ku/ldab those of one class; the
-  // right-hand sides and solutions in work are stored class by class
-  // (work stride wst >= ncls*Tc) and mapped back through col_pos.
-  int ncls, Tc, wst;
+  // class split (SystemOps::ncls == 2): kl/ku/ldab are those of one class, Tc its rows
+  int ncls, Tc;
   const int* row_pos;    // [T] class position of an equation row (null: unsplit)
-  const int* col_pos;    // [T] class position of a variable column (null: unsplit)
-  const unsigned char* colflip_cls;  // [ncls*Tc] colflip in class order
-  DevEll Lp;             // L with its columns in class positions (= L when unsplit)
   // block solve (class split): a unit is one factorisation, shared by the systems
   // (kx, ky) and (kx, -ky) when the recipe has the ky mirror symmetry; a group is
   // upw units (16 with the symmetry, else 32) of one class, 32 lanes = the

@@ -1406,41 +1406,30 @@ __device__ __forceinline__ double2 shfl2(double2 v, int src) {
   return make_double2(__shfl_sync(0xffffffffu, v.x, src), __shfl_sync(0xffffffffu, v.y, src));
 }
 
-// H = lanes per system class: H = 32 for an unsplit system, H = 16 for a class
-// split, the two classes of one system side by side in the two half-warps, in
-// lockstep over their Tc columns (positions p = lane (mod H) of the half; the
-// window bounds become kl <= H-1 and kl+ku <= 2H-1).
-template <int H>
 __global__ void __launch_bounds__(kWPBr * 32) k_subst_real(SolveArgs a) {
-  constexpr int NC = 32 / H;            // classes per warp
-  constexpr int LH = (H == 32) ? 5 : 4;  // log2(H)
+  constexpr int H = 32, LH = 5;  // lanes, log2
   extern __shared__ double smr[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int hl = lane & (H - 1);         // lane within the class's half
-  const int cls = lane >> LH;
-  const int hb = lane - hl;              // first lane of the half
   const int act = blockIdx.x * kWPBr + warp;  // active systems only
   if (act >= a.nact) return;
-  const int T = a.Tc;
+  const int T = a.T;
   const int sid = a.act_list[act];
-  double2* x = a.work + (size_t)sid * a.wst + (size_t)cls * T;  // right-hand side in, solution out
+  double2* x = a.work + (size_t)sid * T;  // right-hand side in, solution out
   {
     const int kl = a.kl, kv = a.kl + a.ku, ldab = a.ldab;
-    const size_t cstr = (size_t)NC * ldab;  // factor column stride (both classes)
-    const double* ab = a.abr + (size_t)act * T * cstr;
-    const unsigned char* dp = a.dpiv + ((size_t)act * NC + cls) * ((T + 7) & ~7);
-    const unsigned char* cflip = a.colflip_cls + (size_t)cls * T;
+    const double* ab = a.abr + (size_t)act * T * ldab;
+    const unsigned char* dp = a.dpiv + (size_t)act * ((T + 7) & ~7);
+    const unsigned char* cflip = a.colflip;
     // Factor columns stream through a per-warp shared-memory ring (kNBUF chunks
     // of kCW columns) with cp.async, kNBUF-1 chunks ahead of the sweep; the
     // forward sweep copies only the L rows of each column, the backward sweep
     // only the U rows.  (ldab is even, so both row ranges are 16-byte aligned.)
     double* ring = smr + (size_t)warp * kNBUF * kCW * a.ring_cols;
-    const int rc = a.ring_cols / NC;                  // ring doubles per class and column
     const int u_rows = (kv + 2) & ~1;                 // rows [0, u_rows) hold U (+ maybe one L row)
     const int l_row0 = (kv + 1) & ~1;                 // rows [l_row0, l_row1) hold L
     const int l_rows = ((kv + 1 + kl + 1) & ~1) - l_row0;
     // ================= forward: P and L =================
-    // lane l owns the positions p = l (mod H); the active window is [j, j+kl].
+    // lane l owns the positions p = l (mod 32); the active window is [j, j+kl].
     // Vector traffic moves in blocks of H columns: the owner of column j takes
     // the new position j+H (loaded one block ahead) and parks y_j until the
     // block's coalesced store.
@@ -1450,45 +1439,45 @@ __global__ void __launch_bounds__(kWPBr * 32) k_subst_real(SolveArgs a) {
         if (c < nchunks) {
           const int j0 = c * kCW, nc = min(kCW, T - 1 - j0);
           double* dst = ring + (size_t)(c % kNBUF) * kCW * a.ring_cols;
-          const int per = l_rows / 2;  // 16-byte pieces per column and class
-          for (int e = lane; e < nc * NC * per; e += 32) {
-            const int q = e / (NC * per), rem = e - q * (NC * per), cc = rem / per, r = rem - cc * per;
-            cp_async16(dst + q * a.ring_cols + cc * rc + 2 * r, ab + (size_t)(j0 + q) * cstr + cc * ldab + l_row0 + 2 * r);
+          const int per = l_rows / 2;  // 16-byte pieces per column
+          for (int e = lane; e < nc * per; e += 32) {
+            const int q = e / per, r = e - q * per;
+            cp_async16(dst + q * a.ring_cols + 2 * r, ab + (size_t)(j0 + q) * ldab + l_row0 + 2 * r);
           }
         }
         cp_async_commit();
       };
 #pragma unroll
       for (int c = 0; c < kNBUF - 1; ++c) issue(c);
-      double2 w = (hl < T) ? x[hl] : zero2();
-      double2 incCur = (H + hl < T) ? x[H + hl] : zero2();
+      double2 w = (lane < T) ? x[lane] : zero2();
+      double2 incCur = (H + lane < T) ? x[H + lane] : zero2();
       double2 incNext = zero2(), ysave = zero2();
-      // pivot offsets of a chunk as two 32-bit words, uniform over the half (rows padded to 8 bytes)
+      // pivot offsets of a chunk as two 32-bit words, uniform over the warp (rows padded to 8 bytes)
       uint2 pw = *reinterpret_cast<const uint2*>(dp);
       for (int c = 0; c < nchunks; ++c) {
         const int j0 = c * kCW;
         if ((j0 & (H - 1)) == 0)  // new block of H columns: next block's incoming values
-          incNext = (j0 + 2 * H + hl < T) ? x[j0 + 2 * H + hl] : zero2();
+          incNext = (j0 + 2 * H + lane < T) ? x[j0 + 2 * H + lane] : zero2();
         const uint2 pwc = pw;
         if (c + 1 < nchunks) pw = *reinterpret_cast<const uint2*>(dp + j0 + kCW);
         __syncwarp();
         issue(c + kNBUF - 1);
         cp_async_wait<kNBUF - 1>();
         __syncwarp();
-        const double* cb = ring + (size_t)(c % kNBUF) * kCW * a.ring_cols + cls * rc;
+        const double* cb = ring + (size_t)(c % kNBUF) * kCW * a.ring_cols;
 #pragma unroll
         for (int q = 0; q < kCW; ++q) {
           const int j = j0 + q;
           if (j < T - 1) {
-            const int src = hb + (j & (H - 1));
-            const int i = (hl - j) & (H - 1);
+            const int src = (j & (H - 1));
+            const int i = (lane - j) & (H - 1);
             const int lm = min(kl, T - 1 - j);
             const double lv = (i >= 1 && i <= lm) ? cb[q * a.ring_cols + (kv + i - l_row0)] : 0.0;
             const int jp = ((q < 4 ? pwc.x : pwc.y) >> (8 * (q & 3))) & 0xFF;
             // Row interchange j <-> j+jp and broadcast of the pivot row in one shuffle:
             // the owner of row j+jp fetches row j (its new content), every other lane
             // fetches the pivot row; the owner of j+jp already holds the pivot value.
-            const int r2 = hb + ((j + jp) & (H - 1));
+            const int r2 = ((j + jp) & (H - 1));
             const bool mine = (jp != 0 && lane == r2);
             const double2 got = shfl2(w, mine ? src : r2);
             const double2 bj = mine ? w : got;
@@ -1500,7 +1489,7 @@ __global__ void __launch_bounds__(kWPBr * 32) k_subst_real(SolveArgs a) {
               w = incCur;
             }
             if ((j & (H - 1)) == H - 1) {  // end of a block of H columns
-              x[j - (H - 1) + hl] = ysave;
+              x[j - (H - 1) + lane] = ysave;
               incCur = incNext;
             }
           }
@@ -1510,18 +1499,18 @@ __global__ void __launch_bounds__(kWPBr * 32) k_subst_real(SolveArgs a) {
       // the last (partial) block of y values and y[T-1]
       const int base = ((T - 1) >> LH) << LH;
       if ((T - 1) & (H - 1)) {
-        if (base + hl <= T - 2) x[base + hl] = ysave;
+        if (base + lane <= T - 2) x[base + lane] = ysave;
       }
-      if (hl == ((T - 1) & (H - 1))) x[T - 1] = w;
+      if (lane == ((T - 1) & (H - 1))) x[T - 1] = w;
     }
     __syncwarp();
     // ================= backward: U (kl+ku super-diagonals, reciprocal diagonal) =================
-    // lane l owns p = l (mod H) in two registers: w0 for (p/H) even, w1 for odd.
+    // lane l owns p = l (mod 32) in two registers: w0 for (p/H) even, w1 for odd.
     // Blocks of H columns j = T-1-H*b-s; the owner of j takes position j-2H.
     {
       double2 w0 = zero2(), w1 = zero2();
       {
-        const int ih = (T - 1 - hl) & (H - 1), ph = T - 1 - ih, pl = ph - H;
+        const int ih = (T - 1 - lane) & (H - 1), ph = T - 1 - ih, pl = ph - H;
         if (ph >= 0) { if ((ph >> LH) & 1) w1 = x[ph]; else w0 = x[ph]; }
         if (pl >= 0) { if ((pl >> LH) & 1) w1 = x[pl]; else w0 = x[pl]; }
       }
@@ -1531,9 +1520,9 @@ __global__ void __launch_bounds__(kWPBr * 32) k_subst_real(SolveArgs a) {
           const int jhi = T - 1 - c * kCW, jlo = max(0, jhi - kCW + 1), nc = jhi - jlo + 1;
           double* dst = ring + (size_t)(c % kNBUF) * kCW * a.ring_cols;
           const int per = u_rows / 2;
-          for (int e = lane; e < nc * NC * per; e += 32) {
-            const int q = e / (NC * per), rem = e - q * (NC * per), cc = rem / per, r = rem - cc * per;  // q counts down from jhi
-            cp_async16(dst + q * a.ring_cols + cc * rc + 2 * r, ab + (size_t)(jhi - q) * cstr + cc * ldab + 2 * r);
+          for (int e = lane; e < nc * per; e += 32) {
+            const int q = e / per, r = e - q * per;  // q counts down from jhi
+            cp_async16(dst + q * a.ring_cols + 2 * r, ab + (size_t)(jhi - q) * ldab + 2 * r);
           }
         }
         cp_async_commit();
@@ -1543,7 +1532,7 @@ __global__ void __launch_bounds__(kWPBr * 32) k_subst_real(SolveArgs a) {
       for (int c = 0; c < kNBUF - 1; ++c) issue(c);
       auto own_col = [&](int b) {  // column of block b finished by this lane (may be < 0)
         const int top = T - 1 - H * b;
-        return top - ((top - hl) & (H - 1));
+        return top - ((top - lane) & (H - 1));
       };
       int jl = own_col(0);
       double2 incCur = (jl - 2 * H >= 0) ? x[jl - 2 * H] : zero2();
@@ -1561,15 +1550,15 @@ __global__ void __launch_bounds__(kWPBr * 32) k_subst_real(SolveArgs a) {
         issue(c + kNBUF - 1);
         cp_async_wait<kNBUF - 1>();
         __syncwarp();
-        const double* cb = ring + (size_t)(c % kNBUF) * kCW * a.ring_cols + cls * rc;
+        const double* cb = ring + (size_t)(c % kNBUF) * kCW * a.ring_cols;
 #pragma unroll
         for (int q = 0; q < kCW; ++q) {
           const int k = k0 + q;
           const int j = T - 1 - k;
           if (j >= 0) {
-            const int src = hb + (j & (H - 1)), sel = (j >> LH) & 1;
+            const int src = (j & (H - 1)), sel = (j >> LH) & 1;
             const double* col = cb + q * a.ring_cols;
-            const int ih = (j - hl) & (H - 1), il = ih + H;
+            const int ih = (j - lane) & (H - 1), il = ih + H;
             const double h = (ih >= 1 && ih <= kv) ? col[kv - ih] : 0.0;
             const double l_ = (il <= kv) ? col[kv - il] : 0.0;
             const double d = col[kv];
@@ -2453,7 +2442,7 @@ __global__ void __launch_bounds__(kRhsThreads) k_rhs_nl(SolveArgs a, NLArgs n) {
           const int pos = a.row_pos[t], c = pos >= a.Tc ? 1 : 0;
           store_block_rhs(a, a.slot[sid], c, pos - c * a.Tc, a.row_neg[t], b);
         } else {
-          a.work[(size_t)sid * a.wst + (a.row_pos ? a.row_pos[t] : t)] = b;
+          a.work[(size_t)sid * T + t] = b;
         }
       } else {
         const double2 v = a.last_stage ? zero2() : b;
@@ -2481,7 +2470,7 @@ __global__ void __launch_bounds__(kRhsThreads) k_kstd_out(SolveArgs a) {
   // only K_std remains (L with its original columns); whole-system solve: the
   // solution is in work (class order = original order), copied to out here
   const bool in_out = a.work2 != nullptr;
-  const DevEll& L = in_out ? a.L : a.Lp;
+  const DevEll& L = a.L;
   for (int e = threadIdx.x; e < ns * kMaxGroups; e += blockDim.x) {
     const int s = e / kMaxGroups, g = e - s * kMaxGroups, sid = a.act_list[a0 + s];
     const int kx = sid / a.d.NYA, ky = sid - kx * a.d.NYA;
@@ -2489,7 +2478,7 @@ __global__ void __launch_bounds__(kRhsThreads) k_kstd_out(SolveArgs a) {
   }
   for (int s = 0; s < ns; ++s) {
     const int sid = a.act_list[a0 + s];
-    const double2* x = in_out ? a.out + (size_t)sid * T : a.work + (size_t)sid * a.wst;
+    const double2* x = in_out ? a.out + (size_t)sid * T : a.work + (size_t)sid * T;
     for (int p = threadIdx.x; p < T; p += blockDim.x) xs[s * T + p] = x[p];
   }
   __syncthreads();
@@ -3750,8 +3739,8 @@ void launch_subst(const SolveArgs& a, cudaStream_t s) {
   }
   // whole systems (no class split): one warp per system
   const size_t sm = (size_t)kWPBr * kNBUF * kCW * a.ring_cols * sizeof(double);
-  set_smem(k_subst_real<32>, sm);
-  k_subst_real<32><<<(a.nact + kWPBr - 1) / kWPBr, kWPBr * 32, sm, s>>>(a);
+  set_smem(k_subst_real, sm);
+  k_subst_real<<<(a.nact + kWPBr - 1) / kWPBr, kWPBr * 32, sm, s>>>(a);
 }
 bool subst_multi_supported(const SolveArgs& a) {
   return a.work2 && a.ngrp > 0 && a.kl == 9 && a.kl + a.ku == 23;

@@ -2824,7 +2824,7 @@ int coral_run(coral_handle* h, int nsteps, const char* output_directory) {
 // Ensembles: many independent plane-layer runs (different grids, parameters
 // and recipes) advanced together on one stream, one CUDA graph per step.  Per
 // stage every member's transforms and right-hand sides are queued, then the
-// band substitutions of all members run as one persistent launch
+// band substitutions of all members run as one launch
 // (k_subst_block_multi), then every member's K_std and mean systems.  The
 // reference solves its systems one (kx, ky) at a time in a loop
 // (src/plane_layer/PL_algebra_z_3D.f90:197-214) and runs one problem per job.

@@ -302,7 +302,7 @@ void launch_solve_real(const SolveArgs& a, const NLArgs& n, cudaStream_t s);
 void launch_rhs_nl(const SolveArgs& a, const NLArgs& n, cudaStream_t s);
 void launch_subst(const SolveArgs& a, cudaStream_t s);
 void launch_kstd_out(const SolveArgs& a, cudaStream_t s);
-// the substitutions of several systems in one persistent launch (ensembles):
+// the substitutions of several systems in one launch (ensembles):
 // d_args[m] the SolveArgs of member m, d_prefix[m] its first group in the
 // concatenated range (d_prefix[nmem] = total); every member must pass
 // subst_multi_supported (block layout, band (9, 23)); wide: some member's groups

@@ -1972,8 +1972,10 @@ __global__ void __launch_bounds__(256) k_pack_back(FactorArgs a, int g0, int gn)
 // column order, the order in which the column sweep reaches it); the solution,
 // scaled back, goes straight into the stage output.
 //
-// What bounds it: the factor and vector streams on large grids, the chain of 2 Tc
-// dependent column steps on small ones.  So (a) the systems (kx, ky) and
+// What bounds it: the factor and vector streams on large grids; on small ones the 2 Tc
+// column steps one after the other, each of them one warp's own instructions (128^2 x
+// 192: 3.4 warps an SM, a scheduler issues in 38% of the cycles, its warp stalls on
+// fixed latencies, 1.1 cycles an instruction, and hardly on memory, 0.3).  So (a) the systems (kx, ky) and
 // (kx, -ky) share one factorisation where the recipe's mirror symmetry allows: 16
 // units a warp, two right-hand sides each, half the factor bytes; (b) the factors
 // come as linear streams of the entries that are nonzero in some unit (k_pack);
@@ -1981,7 +1983,8 @@ __global__ void __launch_bounds__(256) k_pack_back(FactorArgs a, int g0, int gn)
 // with cp.async into a ring in shared memory DF (forward) or DB (backward)
 // columns ahead, so that a column step waits for shared memory only.  Against
 // one thread per system that loads its factors one column ahead, no-slip
-// convection, per launch: 384^2 x 192 3.83 -> 2.42 ms (14.1 GB, 5.8 TB/s),
+// convection, per launch: 384^2 x 192 3.83 -> 2.41 ms (11.65 GB, 6.2 of them the
+// streams, 4.84 TB/s, 0.74 of the copy rate; before, 20.1 GB, 14.7 of factors),
 // 128^2 x 192 1.26 -> 0.39 ms, 64^2 x 48 0.318 -> 0.099 ms; without the symmetry
 // (rotating, 192^2 x 96) 0.72 -> 0.49 ms.
 //

@@ -1,6 +1,6 @@
 """Python mirror of the ensemble C-ABI (coral_ensemble_* in include/coral_b200.h):
 many independent plane-layer runs advanced together, one CUDA graph per step,
-the band substitutions of all members in one persistent launch per stage."""
+the band substitutions of all members in one launch per stage."""
 import ctypes
 
 from . import _lib

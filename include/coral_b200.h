@@ -352,7 +352,7 @@ int coral_set_penalisation_mask(coral_handle* h, const double* mask);
  * coral.parameters.in text: grid, parameters and recipe may differ; the IMEX
  * scheme's stage count may not) advanced together on one CUDA stream with one
  * CUDA graph per step.  Per stage the band substitutions of every member's
- * (kx, ky) systems run as one persistent launch when every member's systems
+ * (kx, ky) systems run as one launch when every member's systems
  * use the split block layout with the plane-layer band (9, 23)
  * (coral_ensemble_query(e, 2) = 1); otherwise member by member.  The
  * reference runs one problem per job and solves its systems one at a time

@@ -53,7 +53,7 @@ struct NetDev {
 // BF16 as they are; an FP32 activation (or gradient) is the exact sum of three
 // BF16 numbers, h = bf16(h) + bf16(rest) + bf16(rest), so h W is three BF16
 // products with FP32 accumulation.  (Relative error of tau against FP64, rms, for
-// inputs of 1 | 0.1 | 0.01 | 1e-5: 1.5e-7 | 1.8e-7 | 1.9e-7 | 1.9e-7; of scalar FP32
+// inputs of 1 | 0.1 | 0.01 | 1e-5: 1.5e-7 | 1.8e-7 | 2.0e-7 | 1.9e-7; of scalar FP32
 // sums in one chain 2.8e-7 | 3.3e-7 | 3.1e-7 | 3.1e-7.)
 //
 // A warp takes 16 points through all layers with its activations in registers: the
